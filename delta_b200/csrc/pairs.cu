@@ -5,6 +5,8 @@
 // and writes 7 more, so the loads and stores are fully coalesced.  Replaces the
 // per-pair loops of bf()/penalty() (bf.cpp:95-118, penalty.cpp:187-210) and the SIMD
 // pair-list kernels ispc_bf / ispc_pen (bf.ispc:3, penalty.ispc:154).
+#include <type_traits>
+
 #include "internal.h"
 #include "tri_cert.cuh"
 #include "tri_gjk.cuh"
@@ -15,7 +17,8 @@ namespace delta {
 enum { M_BF = 0, M_PENALTY = 1, M_PENALTY_ITER = 2, M_GJK = 3, M_HYBRID_PAIR = 4, M_BF_CERT = 5 };
 
 // Launch bounds of the pair kernel: the FP64 bfSolver kernel is held to 96 registers (5
-// blocks of 128 per SM; 109 unbounded, with one 256-thread block fewer per SM), the
+// blocks of 128 per SM; 109 unbounded, with one 256-thread block fewer per SM), FP64 GJK to
+// 128 (2^22 pairs: 1.29 ms unbounded, 1.02 at 3 blocks, 1.00 at 4, 1.11 at 5), the
 // others keep their registers.
 template <class R, int M>
 struct PairBounds {
@@ -24,6 +27,10 @@ struct PairBounds {
 template <>
 struct PairBounds<xf64, M_BF> {
   static constexpr int kThreads = 128, kMinBlocks = 5;
+};
+template <>
+struct PairBounds<xf64, M_GJK> {
+  static constexpr int kThreads = 128, kMinBlocks = 4;
 };
 
 // A warp walks the list 32 pairs at a time and meets at __syncwarp after each group: the
@@ -72,6 +79,65 @@ __global__ void __launch_bounds__(PairBounds<R, M>::kThreads, PairBounds<R, M>::
     }
     dist[i] = to_f64(pq_distance(pq));
     if (flags) flags[i] = (uint8_t)flag;
+    __syncwarp();
+  }
+}
+
+// FP32 GJK.  The iteration counts are heavy-tailed there (mean about 6; 7% of the
+// microbenchmark's pairs take more than 10, up to 36), so with one pair per lane a warp ran
+// for its slowest pair.  Here a warp owns `per_warp` consecutive pairs, and lanes that are
+// done wait only until kGjkRefill of them are; these write their results and take the
+// warp's next pairs.  2^22 pairs: 18.4 ms with the simplex indexed in local memory and
+// always 36 iterations, 1.91 ms with registers and repeated states left out, 1.01 ms here.
+// (In FP64 the counts are even, 3 to 7, and the plain loop is faster: 1.00 against 1.53 ms.)
+constexpr int kGjkRefill = 12;
+constexpr int kGjkThreads = 128;
+__global__ void __launch_bounds__(kGjkThreads)
+    k_pairs_gjk32(int64_t n, int64_t per_warp, const double *__restrict__ a, const double *__restrict__ b, int64_t ld,
+                  double *__restrict__ p, double *__restrict__ q, double *__restrict__ dist,
+                  uint8_t *__restrict__ flags) {
+  const int lane = threadIdx.x & 31;
+  int64_t next = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp;
+  const int64_t end = next + per_warp < n ? next + per_warp : n;
+  if (next >= end) return;
+  float A[3][3], B[3][3];
+  Gjk<float> g;
+  int64_t i = -1;  // this lane's pair
+  bool more = false;
+  for (;;) {
+    const unsigned idle = __ballot_sync(0xffffffffu, !more);
+    if (__popc(idle) >= kGjkRefill || next >= end) {
+      if (!more) {
+        if (i >= 0) {
+          float pq[6];
+          g.points(A, B, pq);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            p[k * ld + i] = to_f64(pq[k]);
+            q[k * ld + i] = to_f64(pq[3 + k]);
+          }
+          dist[i] = to_f64(pq_distance(pq));
+          if (flags) flags[i] = 0;
+        }
+        i = next + __popc(idle & ((1u << lane) - 1u));
+        if (i < end) {
+#pragma unroll
+          for (int v = 0; v < 3; ++v)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              A[v][k] = from_f64<float>(__ldg(a + (3 * v + k) * ld + i));
+              B[v][k] = from_f64<float>(__ldg(b + (3 * v + k) * ld + i));
+            }
+          more = g.start(A, B);
+        } else {
+          i = -1;
+        }
+      }
+      __syncwarp();
+      next += __popc(idle);
+      if (__all_sync(0xffffffffu, i < 0)) return;
+    }
+    if (more) more = g.step(A, B);
     __syncwarp();
   }
 }
@@ -175,6 +241,25 @@ static cudaError_t launch_one(cudaStream_t s, int64_t n, const double *a, const 
   return cudaGetLastError();
 }
 
+// Pairs of a warp of k_pairs_gjk32: enough warps for one wave of 16 per SM, in whole
+// groups of 32; at most 512 (262,143 pairs: 117 us with 96 a warp, 148 with 64, 144 with
+// 256; 2^22: 1.01 ms with 512, 1.28 with 128, 1.07 with 1024).
+static cudaError_t launch_gjk32(cudaStream_t s, int64_t n, const double *a, const double *b, int64_t ld, double *p,
+                                double *q, double *dist, uint8_t *flags, PairLaunch cfg) {
+  const int threads = cfg.threads == 64 ? 64 : kGjkThreads, warps = threads / 32;
+  int64_t per = n / (16 * kNumSMs);
+  if (per > 512) per = 512;
+  if (cfg.blocks_per_sm > 0) {
+    const int64_t least = n / ((int64_t)kNumSMs * cfg.blocks_per_sm * warps);
+    if (per < least) per = least;
+  }
+  per = (per / 32 > 0 ? per / 32 : 1) * 32;
+  int64_t blocks = (n + warps * per - 1) / (warps * per);
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+  k_pairs_gjk32<<<(unsigned)(blocks > 0 ? blocks : 1), threads, 0, s>>>(n, per, a, b, ld, p, q, dist, flags);
+  return cudaGetLastError();
+}
+
 template <class R>
 static cudaError_t launch_prec(int method, cudaStream_t s, int64_t n, const double *a, const double *b, int64_t ld,
                                double me, double *p, double *q, double *dist, uint8_t *flags, PairLaunch cfg) {
@@ -182,7 +267,9 @@ static cudaError_t launch_prec(int method, cudaStream_t s, int64_t n, const doub
     case M_BF: return launch_one<R, M_BF>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
     case M_PENALTY: return launch_one<R, M_PENALTY>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
     case M_PENALTY_ITER: return launch_one<R, M_PENALTY_ITER>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
-    case M_GJK: return launch_one<R, M_GJK>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
+    case M_GJK:
+      if constexpr (std::is_same_v<R, float>) return launch_gjk32(s, n, a, b, ld, p, q, dist, flags, cfg);
+      else return launch_one<R, M_GJK>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
     case M_HYBRID_PAIR: return launch_one<R, M_HYBRID_PAIR>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
     default: return cudaErrorInvalidValue;
   }

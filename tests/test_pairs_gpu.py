@@ -218,3 +218,32 @@ def test_autotuned_launch_keeps_results(ctx, oracle, workload):
 
     with pytest.raises(DeltaError, match="INVALID"):
         set_launch(ctx, 0, 0, 256, 32)  # the FP64 bf kernel takes at most 128 threads per block
+
+
+@pytest.mark.parametrize("scale", [1e6, 1e10, 1e14])
+def test_gjk_repeated_simplices_bit_exact_vs_oracle(ctx, oracle, scale):
+    """Coordinates so large that rounding keeps the error bound above the absolute tolerance
+    1e-6: the reference repeats simplices until its 36th iteration, the kernel leaves whole
+    cycles out.  Same arithmetic, so bit for bit."""
+    from delta_b200.scenarios import narrowphase_pairs
+
+    a, b, _, _ = narrowphase_pairs(20_011, seed=77)
+    gp, gq, gd, _ = _run(ctx, 3, a * scale, b * scale)
+    op, oq, od, _ = oracle.pairs(3, a * scale, b * scale)
+    assert not (_differ(gp, op) | _differ(gq, oq) | _differ(gd[None], od[None])).any()
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 129, 4097, 151_553])
+def test_f32_gjk_does_not_depend_on_the_split(ctx, workload, n):
+    """FP32 GJK takes warps' pairs in the order their lanes fall idle: a pair's result is the
+    same whatever list it stands in (151,553 pairs: 64 a warp, an odd remainder)."""
+    from delta_b200.narrowphase import Context, set_launch
+
+    a, b = (np.tile(x, 3)[:, :n] for x in workload)
+    got = _run(ctx, 3, a, b, precision=1)
+    other = Context(0)
+    set_launch(other, 3, 1, 64, 1)  # few blocks, longer runs of pairs a warp
+    ref = _run(other, 3, np.tile(workload[0], 4), np.tile(workload[1], 4), precision=1)
+    other.close()
+    for x, y in zip(got, ref):
+        assert np.array_equal(x, y[..., :n], equal_nan=x.dtype.kind == "f")
