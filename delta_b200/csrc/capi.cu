@@ -242,7 +242,7 @@ delta_status delta_autotune_pairs(delta_ctx *ctx, int method, int precision, int
   } else {
     for (int t : {64, 128, 256})
       for (int b : {4, 8, 16, 32, 0})  // 0: one thread per pair
-        if (t <= pair_max_threads(method, precision)) cand.push_back(PairLaunch{t, b});
+        if (t <= pair_kernel_threads(method, precision)) cand.push_back(PairLaunch{t, b});
   }
   cudaEvent_t e0, e1;
   cudaError_t e = cudaEventCreate(&e0);

@@ -12,27 +12,24 @@ namespace delta {
 
 constexpr int kNumSMs = 148;  // B200
 
-// Launch shape of a pair-list kernel: threads per block (64, 128, 256) and the grid
-// cap in blocks per SM (cert: in units of the occupancy limit).
-// Launch shape of a pair kernel: threads per block and the grid cap in blocks per SM
-// (0: no cap, one thread per pair).
+// Launch shape of a pair kernel: threads per block (64, 128, 256) and the grid cap in
+// blocks per SM (0: no cap, one thread per pair; cert: in units of the occupancy limit).
+// Blocks of 128: in FP32 (2^22 pairs) hybrid 196 us against 221 with 256, penalty 183
+// against 187, adaptive penalty 218 against 223; the FP64 kernels take at most 128.
 struct PairLaunch {
-  int threads = 256;
+  int threads = 128;
   int blocks_per_sm = 32;
 };
 inline PairLaunch default_pair_launch(int method) {
   PairLaunch c;
-  if (method == 5) {
-    c.threads = 128;
-    c.blocks_per_sm = 8;
-  } else if (method == 0) {
-    c.threads = 128;
-    c.blocks_per_sm = 0;
-  }
+  if (method == 5) c.blocks_per_sm = 8;
+  else if (method == 0) c.blocks_per_sm = 0;
   return c;
 }
-// The largest threads per block the pair kernel of (method, precision) takes (pairs.cu).
+// The largest threads per block a caller may ask of (method, precision), and the largest its
+// kernel is launched with (pairs.cu; a larger request is cut to that).
 int pair_max_threads(int method, int precision);
+int pair_kernel_threads(int method, int precision);
 // Position of coordinate c (0..17: a's 9, then b's 9) of list entry j in the exact
 // solver's staging buffer: tiles of 32 entries, each tile 18 rows of 32 doubles, so one
 // warp's 32 consecutive entries read one contiguous 4.6 KB tile (rather than 18 planes a

@@ -18,8 +18,12 @@ enum { M_BF = 0, M_PENALTY = 1, M_PENALTY_ITER = 2, M_GJK = 3, M_HYBRID_PAIR = 4
 
 // Launch bounds of the pair kernel: the FP64 bfSolver kernel is held to 96 registers (5
 // blocks of 128 per SM; 109 unbounded, with one 256-thread block fewer per SM), FP64 GJK to
-// 128 (2^22 pairs: 1.29 ms unbounded, 1.02 at 3 blocks, 1.00 at 4, 1.11 at 5), the
-// others keep their registers.
+// 128 (2^22 pairs: 1.29 ms unbounded, 1.02 at 3 blocks, 1.00 at 4, 1.11 at 5).  The FP64
+// penalty kernels are bound by the FP64 pipe (44 divisions a pair) once enough warps are
+// resident: unbounded (144-176 registers) one block of 256 fitted an SM.  2^22 pairs,
+// before / 2 / 3 / 4 / 5 blocks of 128 per SM: penalty 549 / 412 / 412 / 381 / 415 us,
+// adaptive penalty 693 / 520 / 520 / 493 / 513, hybrid 551 / 529 / 416 / 433 / 559.  The
+// FP32 kernels keep their registers.
 template <class R, int M>
 struct PairBounds {
   static constexpr int kThreads = 256, kMinBlocks = 1;
@@ -27,6 +31,18 @@ struct PairBounds {
 template <>
 struct PairBounds<xf64, M_BF> {
   static constexpr int kThreads = 128, kMinBlocks = 5;
+};
+template <>
+struct PairBounds<xf64, M_PENALTY> {
+  static constexpr int kThreads = 128, kMinBlocks = 4;
+};
+template <>
+struct PairBounds<xf64, M_PENALTY_ITER> {
+  static constexpr int kThreads = 128, kMinBlocks = 4;
+};
+template <>
+struct PairBounds<xf64, M_HYBRID_PAIR> {
+  static constexpr int kThreads = 128, kMinBlocks = 3;
 };
 template <>
 struct PairBounds<xf64, M_GJK> {
@@ -292,6 +308,10 @@ static cudaError_t launch_cert(cudaStream_t s, int64_t n, const double *a, const
 int pair_max_threads(int method, int precision) {
   if (method == M_BF_CERT) return 128;
   return (method == M_BF && precision == 0) ? PairBounds<xf64, M_BF>::kThreads : 256;
+}
+
+int pair_kernel_threads(int method, int precision) {
+  return precision == 0 || method == M_GJK || method == M_BF_CERT ? 128 : 256;
 }
 
 cudaError_t launch_pairs_cfg(int method, int precision, cudaStream_t s, int64_t n, const double *a, const double *b,
