@@ -16,9 +16,7 @@ namespace delta {
 
 enum { M_BF = 0, M_PENALTY = 1, M_PENALTY_ITER = 2, M_GJK = 3, M_HYBRID_PAIR = 4, M_BF_CERT = 5 };
 
-// Launch bounds of the pair kernel: the FP64 bfSolver kernel is held to 96 registers (5
-// blocks of 128 per SM; 109 unbounded, with one 256-thread block fewer per SM), FP64 GJK to
-// 128 (2^22 pairs: 1.29 ms unbounded, 1.02 at 3 blocks, 1.00 at 4, 1.11 at 5).  The FP64
+// Launch bounds of the pair kernel: FP64 GJK is held to 128 registers (2^22 pairs: 1.29 ms unbounded, 1.02 at 3 blocks, 1.00 at 4, 1.11 at 5).  The FP64
 // penalty kernels are bound by the FP64 pipe (44 divisions a pair) once enough warps are
 // resident: unbounded (144-176 registers) one block of 256 fitted an SM.  2^22 pairs,
 // before / 2 / 3 / 4 / 5 blocks of 128 per SM: penalty 549 / 412 / 412 / 381 / 415 us,
@@ -27,10 +25,6 @@ enum { M_BF = 0, M_PENALTY = 1, M_PENALTY_ITER = 2, M_GJK = 3, M_HYBRID_PAIR = 4
 template <class R, int M>
 struct PairBounds {
   static constexpr int kThreads = 256, kMinBlocks = 1;
-};
-template <>
-struct PairBounds<xf64, M_BF> {
-  static constexpr int kThreads = 128, kMinBlocks = 5;
 };
 template <>
 struct PairBounds<xf64, M_PENALTY> {
@@ -96,6 +90,174 @@ __global__ void __launch_bounds__(PairBounds<R, M>::kThreads, PairBounds<R, M>::
     dist[i] = to_f64(pq_distance(pq));
     if (flags) flags[i] = (uint8_t)flag;
     __syncwarp();
+  }
+}
+
+// FP64 bfSolver (bf.cpp:217-1178): the 15 evaluations, comparisons and results of
+// bf_solve_lean.  Both kernels keep the triangles in shared memory (plane, pair) and load a
+// feature's vertices from there, at a row that is the same for the whole warp, in a column
+// of the lane's own: nothing of a pair but the running minimum stays in registers between
+// features (the register copies rotated by bf_solve_lean held 36 doubles).
+struct BfBest {
+  xf64 d, p0, p1;  // distance and the winner's parameters
+  int id;          // edge pair 3 ea + eb; vertex-face 3 face + vertex (face 0: A's)
+  __device__ __forceinline__ void start() {
+    d = xf64(1E+30);
+    p0 = p1 = xf64(0.0);
+    id = 0;
+  }
+  __device__ __forceinline__ void take(xf64 dist, xf64 x0, xf64 x1, int j) {
+    if (dist < d) {
+      d = dist;
+      p0 = x0;
+      p1 = x1;
+      id = j;
+    }
+  }
+};
+
+template <int COLS>
+struct BfTile {
+  double v[18][COLS];
+  __device__ __forceinline__ void vertex(int t, int col, xf64 x[3]) const {  // A's 0..2, B's 3..5
+#pragma unroll
+    for (int k = 0; k < 3; ++k) x[k] = xf64(v[3 * t + k][col]);
+  }
+  // the edge pairs of A's edge ea, in order
+  __device__ __forceinline__ void edges(int ea, int col, BfBest &best) const {
+    xf64 HA[3], TA[3];
+    vertex(ea, col, HA);
+    vertex(ea == 2 ? 0 : ea + 1, col, TA);
+#pragma unroll 1
+    for (int eb = 0; eb < 3; ++eb) {
+      xf64 HB[3], TB[3], sc, tc;
+      vertex(3 + eb, col, HB);
+      vertex(eb == 2 ? 3 : 4 + eb, col, TB);
+      const xf64 d = seg_seg_ref(HA, TA, HB, TB, sc, tc);
+      best.take(d, sc, tc, 3 * ea + eb);
+    }
+  }
+  // the vertices of the other triangle against face 0 (A) or 1 (B), in order
+  __device__ __forceinline__ void faces(int face, int col, BfBest &best) const {
+    xf64 T0[3], T1[3], T2[3];
+    vertex(3 * face, col, T0);
+    vertex(3 * face + 1, col, T1);
+    vertex(3 * face + 2, col, T2);
+#pragma unroll 1
+    for (int j = 0; j < 3; ++j) {
+      xf64 X[3], s, t;
+      vertex(3 * (1 - face) + j, col, X);
+      const xf64 d = pt_tri_ref(T0, T1, T2, X, s, t);
+      best.take(d, s, t, 3 * face + j);
+    }
+  }
+  // the winner's points (seg_seg_points, pt_tri_points) to the outputs of pair i
+  __device__ __forceinline__ void write(int col, const BfBest &e, const BfBest &f, int64_t i, int64_t ld, double *p,
+                                        double *q, double *dist, uint8_t *flags) const {
+    xf64 pq[6];
+    if (f.d > e.d) {
+      const int ea = e.id / 3, eb = e.id % 3;
+      xf64 HA[3], TA[3], HB[3], TB[3];
+      vertex(ea, col, HA);
+      vertex(ea == 2 ? 0 : ea + 1, col, TA);
+      vertex(3 + eb, col, HB);
+      vertex(eb == 2 ? 3 : 4 + eb, col, TB);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        pq[k] = TA[k] + ((HA[k] - TA[k]) * e.p0);
+        pq[3 + k] = TB[k] + ((HB[k] - TB[k]) * e.p1);
+      }
+    } else {
+      const bool onA = f.id < 3;
+      xf64 T0[3], T1[3], T2[3], X[3];
+      vertex(onA ? 0 : 3, col, T0);
+      vertex(onA ? 1 : 4, col, T1);
+      vertex(onA ? 2 : 5, col, T2);
+      vertex(onA ? 3 + f.id : f.id - 3, col, X);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const xf64 face = T0[k] + ((T2[k] - T0[k]) * f.p1) + ((T1[k] - T0[k]) * f.p0);
+        pq[k] = onA ? face : X[k];
+        pq[3 + k] = onA ? X[k] : face;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      p[k * ld + i] = pq[k].v;
+      q[k * ld + i] = pq[3 + k].v;
+    }
+    dist[i] = pq_distance(pq).v;
+    if (flags) flags[i] = 0;
+  }
+};
+
+// A thread per pair, 8 blocks of 128 per SM (64 registers).  Bound by the FP64 pipe and the
+// lanes' divergence: 2^22 pairs 1084 us before, 762 now (92 registers: 808; 48: 859).
+constexpr int kBfThreads = 128;
+__global__ void __launch_bounds__(kBfThreads, 8)
+    k_pairs_bf64(int64_t n, const double *__restrict__ a, const double *__restrict__ b, int64_t ld,
+                 double *__restrict__ p, double *__restrict__ q, double *__restrict__ dist,
+                 uint8_t *__restrict__ flags) {
+  __shared__ BfTile<kBfThreads> tile;
+  const int col = threadIdx.x;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = base + col;
+    if (i < n) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        tile.v[k][col] = __ldg(a + k * ld + i);
+        tile.v[9 + k][col] = __ldg(b + k * ld + i);
+      }
+      BfBest e, f;
+      e.start();
+      f.start();
+#pragma unroll 1
+      for (int ea = 0; ea < 3; ++ea) tile.edges(ea, col, e);
+#pragma unroll 1
+      for (int face = 0; face < 2; ++face) tile.faces(face, col, f);
+      tile.write(col, e, f, i, ld, p, q, dist, flags);
+    }
+    __syncwarp();
+  }
+}
+
+// Short lists: five warps to 32 pairs (a lane per pair), warps 0..2 one edge of A each,
+// warps 3..4 one face each; then the first warp takes the minima in the same order.  A
+// pair's chain of 15 dependent evaluations shrinks to 3.
+constexpr int kBfSplitWarps = 5;
+__global__ void __launch_bounds__(32 * kBfSplitWarps, 6)
+    k_pairs_bf64_split(int64_t n, const double *__restrict__ a, const double *__restrict__ b, int64_t ld,
+                       double *__restrict__ p, double *__restrict__ q, double *__restrict__ dist,
+                       uint8_t *__restrict__ flags) {
+  __shared__ BfTile<32> tile;
+  __shared__ double s_d[kBfSplitWarps][32], s_p0[kBfSplitWarps][32], s_p1[kBfSplitWarps][32];
+  __shared__ uint8_t s_id[kBfSplitWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int64_t base = (int64_t)blockIdx.x * 32; base < n; base += (int64_t)gridDim.x * 32) {
+    const int64_t i = base + lane, ii = i < n ? i : n - 1;
+    for (int k = w; k < 18; k += kBfSplitWarps)
+      tile.v[k][lane] = k < 9 ? __ldg(a + k * ld + ii) : __ldg(b + (k - 9) * ld + ii);
+    __syncthreads();
+    BfBest best;
+    best.start();
+    if (w < 3) tile.edges(w, lane, best);
+    else tile.faces(w - 3, lane, best);
+    s_d[w][lane] = best.d.v;
+    s_p0[w][lane] = best.p0.v;
+    s_p1[w][lane] = best.p1.v;
+    s_id[w][lane] = (uint8_t)best.id;
+    __syncthreads();
+    if (w == 0 && i < n) {
+      BfBest e, f;
+      e.start();
+      f.start();
+#pragma unroll
+      for (int g = 0; g < 3; ++g) e.take(xf64(s_d[g][lane]), xf64(s_p0[g][lane]), xf64(s_p1[g][lane]), s_id[g][lane]);
+#pragma unroll
+      for (int g = 3; g < 5; ++g) f.take(xf64(s_d[g][lane]), xf64(s_p0[g][lane]), xf64(s_p1[g][lane]), s_id[g][lane]);
+      tile.write(lane, e, f, i, ld, p, q, dist, flags);
+    }
+    __syncthreads();
   }
 }
 
@@ -276,11 +438,30 @@ static cudaError_t launch_gjk32(cudaStream_t s, int64_t n, const double *a, cons
   return cudaGetLastError();
 }
 
+// Below this the split kernel is the faster one (us, whole / split): 4,097 pairs 16.9 / 8.8,
+// 20,000 17.0 / 11.7, 65,537 23.1 / 20.3, 98,000 29.3 / 27.2, 131,000 33.4 / 33.4, 196,000
+// 46.9 / 47.7, 262,143 55.9 / 62.1.
+constexpr int64_t kBfSplitPairs = 1 << 17;
+static cudaError_t launch_bf64(cudaStream_t s, int64_t n, const double *a, const double *b, int64_t ld, double *p,
+                               double *q, double *dist, uint8_t *flags, PairLaunch cfg) {
+  const bool split = n < kBfSplitPairs;
+  const int threads = cfg.threads == 64 ? 64 : kBfThreads, pairs = split ? 32 : threads;
+  int64_t blocks = (n + pairs - 1) / pairs;
+  if (cfg.blocks_per_sm > 0 && blocks > (int64_t)kNumSMs * cfg.blocks_per_sm) blocks = (int64_t)kNumSMs * cfg.blocks_per_sm;
+  if (blocks > 0x7fffffffLL) blocks = 0x7fffffffLL;
+  if (blocks < 1) blocks = 1;
+  if (split) k_pairs_bf64_split<<<(unsigned)blocks, 32 * kBfSplitWarps, 0, s>>>(n, a, b, ld, p, q, dist, flags);
+  else k_pairs_bf64<<<(unsigned)blocks, threads, 0, s>>>(n, a, b, ld, p, q, dist, flags);
+  return cudaGetLastError();
+}
+
 template <class R>
 static cudaError_t launch_prec(int method, cudaStream_t s, int64_t n, const double *a, const double *b, int64_t ld,
                                double me, double *p, double *q, double *dist, uint8_t *flags, PairLaunch cfg) {
   switch (method) {
-    case M_BF: return launch_one<R, M_BF>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
+    case M_BF:
+      if constexpr (std::is_same_v<R, float>) return launch_one<R, M_BF>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
+      else return launch_bf64(s, n, a, b, ld, p, q, dist, flags, cfg);
     case M_PENALTY: return launch_one<R, M_PENALTY>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
     case M_PENALTY_ITER: return launch_one<R, M_PENALTY_ITER>(s, n, a, b, ld, me, p, q, dist, flags, cfg);
     case M_GJK:
@@ -307,7 +488,7 @@ static cudaError_t launch_cert(cudaStream_t s, int64_t n, const double *a, const
 
 int pair_max_threads(int method, int precision) {
   if (method == M_BF_CERT) return 128;
-  return (method == M_BF && precision == 0) ? PairBounds<xf64, M_BF>::kThreads : 256;
+  return (method == M_BF && precision == 0) ? kBfThreads : 256;
 }
 
 int pair_kernel_threads(int method, int precision) {

@@ -247,3 +247,22 @@ def test_f32_gjk_does_not_depend_on_the_split(ctx, workload, n):
     other.close()
     for x, y in zip(got, ref):
         assert np.array_equal(x, y[..., :n], equal_nan=x.dtype.kind == "f")
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129, 131_071, 131_072, 131_073])
+def test_f64_bf_on_a_coarse_grid_bit_exact_vs_oracle(ctx, oracle, n):
+    """bfSolver at the edges of its kernels' tiles and on both sides of the length at which
+    it changes from five warps per 32 pairs to a thread per pair.  Vertices on a coarse grid:
+    ties between features, degenerate triangles and every region of the point-triangle
+    distance, its borders included."""
+    from delta_b200.narrowphase import Context
+
+    rng = np.random.default_rng(n)
+    a = rng.integers(0, 5, (9, n)) / 4.0
+    b = rng.integers(0, 5, (9, n)) / 4.0 + np.repeat(rng.integers(0, 3, (1, n)) / 8.0, 9, 0)
+    fresh = Context(0)  # the default launch shape
+    gp, gq, gd, gf = _run(fresh, 0, a, b)
+    fresh.close()
+    op, oq, od, of = oracle.pairs(0, a, b)
+    assert not (_differ(gp, op) | _differ(gq, oq) | _differ(gd[None], od[None])).any()
+    assert np.array_equal(gf, of)
