@@ -17,6 +17,7 @@
 #include "blockscan.cuh"
 #include "internal.h"
 #include "pose.cuh"
+#include "tri_bf64.cuh"
 #include "tri_cert.cuh"
 #include "tri_learned.cuh"
 #include "tri_gjk.cuh"
@@ -54,6 +55,8 @@ struct RawContacts {
   // culled drivers: the body-pair work queue of the culling kernel (zeroed before it runs);
   // null: blocks take the pairs by a fixed stride
   unsigned long long *pair_queue;
+  // culling distance added per unit of the largest coordinate of the two bodies' boxes
+  double rel_slack;
 };
 
 struct DevStats {
@@ -478,12 +481,12 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
     do {  // one body pair; `continue` ends it
     if (rc.pcnt && tid == 0) rc.pcnt[k] = 0;  // the pair's contact count (k_cert_survivors)
     const int32_t a = pa[k], b = pb[k];
-    if (a < 0 || b < 0) continue;
+    // (an index past the bodies is reported by k_check_detect)
+    if (a < 0 || b < 0 || a >= m.n_bodies || b >= m.n_bodies) continue;
     const int64_t tA0 = m.tri_offset[a], tB0 = m.tri_offset[b];
     const int32_t nA = (int32_t)(m.tri_offset[a + 1] - tA0), nB = (int32_t)(m.tri_offset[b + 1] - tB0);
     if (tid == 0) atomicAdd(&st->tri_pairs, (unsigned long long)nA * (unsigned long long)nB);
     const double mg = (xf64(m.eps[a]) + xf64(m.eps[b])).v;
-    const double cull = mg * (1.0 + 1e-9) + 1e-12, cull2 = cull * cull;
     double Alo[3], Ahi[3], Blo[3], Bhi[3];
     const Pose &P = rc.pose;
     if (P.rx) {
@@ -498,6 +501,15 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
         Bhi[c] = rc.bbox ? rc.bbox[6 * (int64_t)b + 3 + c] : INFINITY;
       }
     }
+    double cull = mg * (1.0 + 1e-9) + 1e-12;
+    if (rc.rel_slack > 0.0) {
+      double big = 0.0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        big = fmax(big, fmax(fmax(fabs(Alo[c]), fabs(Ahi[c])), fmax(fabs(Blo[c]), fabs(Bhi[c]))));
+      cull += rc.rel_slack * big;
+    }
+    const double cull2 = cull * cull;
     if (box_gap2(Alo, Ahi, Blo, Bhi) > cull2) continue;
     const bool moveA = P.rx && !P.obstacle[a], moveB = P.rx && !P.obstacle[b];
     if (tid == 0 && moveA) QA = body_pose(P, a);
@@ -599,9 +611,10 @@ __global__ void __launch_bounds__(128, 5) k_cert_survivors(delta_meshes m, const
 // The reference's FP64 bfSolver (bf.cpp:217-1178, xf64) over the survivors of the box
 // test, one per thread: the culled driver without the FP32 filter (DELTA_DRV_BF_CULLED),
 // which separates what the culling gains from what the certified FP32 solver gains.
-__global__ void __launch_bounds__(128, 5) k_bf64_survivors(delta_meshes m, const int32_t *__restrict__ pa,
+__global__ void __launch_bounds__(128, 8) k_bf64_survivors(delta_meshes m, const int32_t *__restrict__ pa,
                                                            const int32_t *__restrict__ pb, RawContacts rc) {
   dep_sync();
+  __shared__ BfTile<128> tile;
   const unsigned long long cnt = *rc.sv_count;
   const int64_t n = (int64_t)cnt < rc.sv_cap ? (int64_t)cnt : rc.sv_cap;
   // a warp takes 32 survivors at a time and meets at __syncwarp after them, so that its
@@ -630,15 +643,15 @@ __global__ void __launch_bounds__(128, 5) k_bf64_survivors(delta_meshes m, const
     double A[3][3], B[3][3], pq[6];
     load_tri_cur(m, rc.pose, a, r.tA, A);
     load_tri_cur(m, rc.pose, b, r.tB0 + tb, B);
-    xf64 A64[3][3], B64[3][3], out[6];
 #pragma unroll
     for (int v = 0; v < 3; ++v)
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        A64[v][k] = xf64(A[v][k]);
-        B64[v][k] = xf64(B[v][k]);
+        tile.v[3 * v + k][threadIdx.x] = A[v][k];
+        tile.v[9 + 3 * v + k][threadIdx.x] = B[v][k];
       }
-    bf_solve_lean(A64, B64, out);
+    xf64 out[6];
+    tile.solve(threadIdx.x, out);
 #pragma unroll
     for (int k = 0; k < 6; ++k) pq[k] = out[k].v;
     const double mg = (xf64(r.epsA) + xf64(r.epsB)).v;
@@ -725,23 +738,26 @@ inline cudaError_t launch_survivors(int driver, cudaStream_t s, const delta_mesh
   return launch_dep(dep, k_cert_survivors, (unsigned)blocks, 128, 0, s, m, pa, pb, rc, st);
 }
 
-__global__ void k_sv_evaluated(const unsigned long long *sv_count, int64_t sv_cap, DevStats *st, int *ovf) {
-  const unsigned long long c = *sv_count;
-  st->evaluated += c;
-  if (ovf && c > (unsigned long long)sv_cap) atomicCAS(ovf, 0, 1);
+// Argument check: bad = 1 for a body index out of range, else 2 for a
+// body of 65536 or more triangles.
+__global__ void k_check_detect(const int64_t *tri_offset, const int32_t *pa, const int32_t *pb, int64_t n_pairs,
+                               int32_t n_bodies, int *bad) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n_pairs && (pa[t] < 0 || pa[t] >= n_bodies || pb[t] < 0 || pb[t] >= n_bodies)) atomicExch(bad, 1);
+  if (t < n_bodies) {
+    const int64_t n = tri_offset[t + 1] - tri_offset[t];
+    if (n < 0 || n >= 65536) atomicCAS(bad, 0, 2);
+  }
 }
 
+// Rows (A triangles) per pair, a zero after the last; 0 for an index out of range, which
+// k_check_detect reports.
 __global__ void k_rows_per_pair(const int64_t *tri_offset, const int32_t *pa, int64_t n_pairs, int32_t n_bodies,
-                                int64_t *rows, int *bad) {
+                                int64_t *rows) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n_pairs) return;
-  const int32_t a = pa[k];
-  if (a < 0 || a >= n_bodies) {
-    atomicExch(bad, 1);
-    rows[k] = 0;
-    return;
-  }
-  rows[k] = tri_offset[a + 1] - tri_offset[a];
+  if (k > n_pairs) return;
+  const int32_t a = k < n_pairs ? pa[k] : -1;
+  rows[k] = a < 0 || a >= n_bodies ? 0 : tri_offset[a + 1] - tri_offset[a];
 }
 
 __global__ void k_rows_fixed(const int64_t *tri_offset, const int32_t *pa, int64_t cap, int64_t *rows) {
@@ -867,21 +883,6 @@ __global__ void k_cert_tail(const unsigned long long *sv_count, int64_t sv_cap, 
   }
 }
 
-__global__ void k_check_pairs(const int64_t *tri_offset, const int32_t *pb, int64_t n_pairs, int32_t n_bodies,
-                              int *bad) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n_pairs) return;
-  const int32_t b = pb[k];
-  if (b < 0 || b >= n_bodies) atomicExch(bad, 1);
-}
-
-__global__ void k_max_tris(const int64_t *tri_offset, int32_t n_bodies, int *bad) {
-  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_bodies) return;
-  const int64_t n = tri_offset[i + 1] - tri_offset[i];
-  if (n < 0 || n >= 65536) atomicExch(bad, 2);
-}
-
 __global__ void k_iota(int64_t *v, int64_t n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) v[i] = i;
@@ -959,34 +960,105 @@ cudaError_t detect_launch_limits(int driver, int *cull_per_sm, int *surv_per_sm)
              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(surv_per_sm, k_cert_survivors, 128, 0);
 }
 
-// Scratch slots used here: 2 rows/row_offset, 3 raw contacts, 4 sort buffers, 5 small state.
-delta_status detect_run(delta_ctx *ctx, int driver, int precision, const delta_meshes &m, const int32_t *pa,
-                        const int32_t *pb, int64_t n_pairs, const delta_contacts *out, int64_t *n_out,
-                        delta_stats *stats, int64_t *counters, const Pose *pose) {
+// The caller's detections' small device state: [0] argument check, then the statistics, the
+// work queue, the contact count and the survivor count.
+struct DetectSmall {
+  int bad;
+  char pad[252];
+  DevStats stats;
+  unsigned long long queue, count, sv_count, unused[5];
+};
+
+// Raw contact buffer of cap entries (scratch slot 3).
+static delta_status raw_contacts(delta_ctx *ctx, int64_t cap, RawContacts &rc) {
+  void *raw = nullptr;
+  const size_t per = 14 * sizeof(double) + 4 * sizeof(int32_t) + 1 + 2 * sizeof(uint64_t);
+  delta_status st = ctx_scratch(ctx, 3, per * (size_t)cap + 64, &raw);
+  if (st != DELTA_OK) return st;
+  rc.cap = cap;
+  rc.f = (double *)raw;
+  rc.key = (uint64_t *)(rc.f + 14 * cap);
+  rc.i = (int32_t *)(rc.key + 2 * cap);
+  rc.fric = (uint8_t *)(rc.i + 4 * cap);
+  return DELTA_OK;
+}
+
+static delta_status bad_argument(int bad) {
+  return set_error(DELTA_ERR_INVALID, bad == 1 ? "delta_detect: body index out of range"
+                                               : "delta_detect: a body has 65536 or more triangles");
+}
+
+// The culled drivers' contacts into rc, unordered: argument check, box culling into the
+// survivor list, the survivors' solver, all enqueued at once (the solver reads the
+// survivors' number on the device); one read-back.  A buffer that was too small is grown
+// and the detection repeated.
+static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes &m, const int32_t *pa,
+                                  const int32_t *pb, int64_t n_pairs, int64_t cap, DetectSmall *dev,
+                                  DetectSmall *host, const Pose *pose, RawContacts &rc) {
   cudaStream_t s = ctx->stream;
   delta_status st;
   cudaError_t e;
-  // small device state: [0] bad flag (int), then DevStats, queue counter, contact counter
-  void *small = nullptr;
-  const size_t small_bytes = 256 + sizeof(DevStats) + 64;
-  if ((st = ctx_scratch(ctx, 5, small_bytes, &small)) != DELTA_OK) return st;
-  int *bad = (int *)small;
-  DevStats *dstats = (DevStats *)((char *)small + 256);
-  unsigned long long *queue = (unsigned long long *)((char *)small + 256 + sizeof(DevStats));
-  unsigned long long *count = queue + 1;
-  unsigned long long *sv_count = queue + 2;
-  if ((e = cudaMemsetAsync(small, 0, small_bytes, s)) != cudaSuccess) return cuda_error(e, "detect memset");
+  if (!cull_stride()) rc.pair_queue = &dev->queue;
+  rc.count = &dev->count;
+  rc.sv_count = &dev->sv_count;
+  if (pose) {
+    rc.pose = *pose;  // current vertices and body boxes from the bodies' poses
+  } else {
+    // body boxes of the current vertices for the culling
+    void *bb = nullptr;
+    if ((st = ctx_scratch(ctx, 23, 48 * (size_t)m.n_bodies + 64, &bb)) != DELTA_OK) return st;
+    const int64_t warps = std::min<int64_t>(m.n_bodies, (int64_t)kNumSMs * 64);
+    k_body_boxes<<<(unsigned)std::max<int64_t>(1, (warps * 32 + 127) / 128), 128, 0, s>>>(m, (double *)bb);
+    ctx->launches += 1;
+    rc.bbox = (const double *)bb;
+  }
+  int64_t sv_cap = 8 * cap > (1 << 16) ? 8 * cap : (1 << 16);
+  for (;;) {
+    if ((st = raw_contacts(ctx, cap, rc)) != DELTA_OK) return st;
+    void *svb = nullptr;
+    if ((st = ctx_scratch(ctx, 9, sizeof(uint64_t) * (size_t)sv_cap, &svb)) != DELTA_OK) return st;
+    rc.sv = (uint64_t *)svb;
+    rc.sv_cap = sv_cap;
+    if ((e = cudaMemsetAsync(dev, 0, sizeof(DetectSmall), s)) != cudaSuccess) return cuda_error(e, "detect memset");
+    const int64_t checks = std::max<int64_t>(n_pairs, m.n_bodies);
+    k_check_detect<<<(unsigned)((checks + 255) / 256), 256, 0, s>>>(m.tri_offset, pa, pb, n_pairs, m.n_bodies,
+                                                                   &dev->bad);
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "detect check");
+    if ((e = launch_cull(s, m, pa, pb, n_pairs, rc, &dev->stats, ctx->cull_blocks_per_sm)) != cudaSuccess)
+      return cuda_error(e, "cull kernel");
+    if ((e = launch_survivors(driver, s, m, pa, pb, rc, &dev->stats, -1, ctx->surv_blocks_per_sm)) != cudaSuccess)
+      return cuda_error(e, "survivor kernel");
+    ctx->launches += 3;
+    if ((e = cudaMemcpyAsync(host, dev, sizeof(DetectSmall), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+      return cuda_error(e, "detect counts");
+    if (host->bad) return bad_argument(host->bad);
+    host->stats.evaluated = host->sv_count;
+    const int64_t nsv = (int64_t)host->sv_count, nc = (int64_t)host->count;
+    if (nsv > sv_cap) sv_cap = nsv + nsv / 4;  // (the contacts of the survivors listed so far: counted again)
+    else if (nc > cap) cap = nc + nc / 4;
+    else return DELTA_OK;
+  }
+}
 
+// The other drivers' contacts into rc, unordered: rows of the triangle pairs of every body
+// pair from a work queue.
+static delta_status detect_rows(delta_ctx *ctx, int driver, int precision, const delta_meshes &m, const int32_t *pa,
+                                const int32_t *pb, int64_t n_pairs, int64_t cap, DetectSmall *dev,
+                                DetectSmall *host, RawContacts &rc) {
+  cudaStream_t s = ctx->stream;
+  delta_status st;
+  cudaError_t e;
+  if ((e = cudaMemsetAsync(dev, 0, sizeof(DetectSmall), s)) != cudaSuccess) return cuda_error(e, "detect memset");
   // rows per pair and their exclusive prefix sum
   void *rbuf = nullptr;
   if ((st = ctx_scratch(ctx, 2, sizeof(int64_t) * (size_t)(2 * n_pairs + 2), &rbuf)) != DELTA_OK) return st;
   int64_t *rows = (int64_t *)rbuf, *row_offset = rows + n_pairs + 1;
-  const unsigned g = (unsigned)((n_pairs + 255) / 256);
-  k_rows_per_pair<<<g, 256, 0, s>>>(m.tri_offset, pa, n_pairs, m.n_bodies, rows, bad);
-  k_check_pairs<<<g, 256, 0, s>>>(m.tri_offset, pb, n_pairs, m.n_bodies, bad);
-  k_max_tris<<<(unsigned)((m.n_bodies + 255) / 256), 256, 0, s>>>(m.tri_offset, m.n_bodies, bad);
-  ctx->launches += 3;
-  if ((e = cudaMemsetAsync(rows + n_pairs, 0, sizeof(int64_t), s)) != cudaSuccess) return cuda_error(e, "memset");
+  const int64_t checks = std::max<int64_t>(n_pairs, m.n_bodies);
+  k_check_detect<<<(unsigned)((checks + 255) / 256), 256, 0, s>>>(m.tri_offset, pa, pb, n_pairs, m.n_bodies,
+                                                                 &dev->bad);
+  k_rows_per_pair<<<(unsigned)((n_pairs + 256) / 256), 256, 0, s>>>(m.tri_offset, pa, n_pairs, m.n_bodies, rows);
+  ctx->launches += 2;
   size_t temp_bytes = 0;
   cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, rows, row_offset, n_pairs + 1, s);
   void *temp = nullptr;
@@ -998,110 +1070,80 @@ delta_status detect_run(delta_ctx *ctx, int driver, int precision, const delta_m
   int hbad = 0;
   if ((e = cudaMemcpyAsync(&total_rows, row_offset + n_pairs, sizeof(int64_t), cudaMemcpyDeviceToHost, s)) !=
           cudaSuccess ||
-      (e = cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(&hbad, &dev->bad, sizeof(int), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
     return cuda_error(e, "detect rows");
-  if (hbad == 1) return set_error(DELTA_ERR_INVALID, "delta_detect: body index out of range");
-  if (hbad == 2) return set_error(DELTA_ERR_INVALID, "delta_detect: a body has 65536 or more triangles");
-
-  // raw contact buffer: at least the caller's capacity; grown and rerun when it overflows
-  int64_t cap = out->capacity > 1024 ? out->capacity : 1024;
-  unsigned long long hcount = 0;
-  RawContacts rc{};
-  rc.tbits = 16;
-  const bool culled = driver == DELTA_DRV_BF_CERT || driver == DELTA_DRV_BF_CULLED || driver == DELTA_DRV_LEARNED;
-  if (culled && !cull_stride()) rc.pair_queue = queue;  // zeroed below before every culling launch
-  if (culled && pose) {
-    rc.pose = *pose;  // current vertices and body boxes from the bodies' poses
-  } else if (culled) {
-    // body boxes of the current vertices for the culling
-    void *bb = nullptr;
-    if ((st = ctx_scratch(ctx, 23, 48 * (size_t)m.n_bodies + 64, &bb)) != DELTA_OK) return st;
-    const int64_t warps = std::min<int64_t>(m.n_bodies, (int64_t)kNumSMs * 64);
-    k_body_boxes<<<(unsigned)std::max<int64_t>(1, (warps * 32 + 127) / 128), 128, 0, s>>>(m, (double *)bb);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "body boxes");
-    ctx->launches += 1;
-    rc.bbox = (const double *)bb;
-  }
+  if (hbad) return bad_argument(hbad);
+  rc.count = &dev->count;
   for (int attempt = 0; attempt < 2; ++attempt) {
-    void *raw = nullptr;
-    const size_t per = 14 * sizeof(double) + 4 * sizeof(int32_t) + 1 + 2 * sizeof(uint64_t);
-    if ((st = ctx_scratch(ctx, 3, per * (size_t)cap + 64, &raw)) != DELTA_OK) return st;
-    rc.cap = cap;
-    rc.f = (double *)raw;
-    rc.key = (uint64_t *)(rc.f + 14 * cap);
-    rc.i = (int32_t *)(rc.key + 2 * cap);
-    rc.fric = (uint8_t *)(rc.i + 4 * cap);
-    rc.count = count;
-    rc.sv_count = sv_count;
-    if ((e = cudaMemsetAsync(queue, 0, 3 * sizeof(unsigned long long), s)) != cudaSuccess)
-      return cuda_error(e, "memset");
-    if ((e = cudaMemsetAsync(dstats, 0, sizeof(DevStats), s)) != cudaSuccess) return cuda_error(e, "memset");
-    if (culled) {
-      // phase 1: box culling into the survivor list (grown and repeated on overflow);
-      // phase 2: the survivors' solver (certified bf, full warps across pairs; or FP64 bf)
-      int64_t sv_cap = 8 * cap > (1 << 16) ? 8 * cap : (1 << 16);
-      unsigned long long hsv = 0;
-      for (int sv_attempt = 0; sv_attempt < 2; ++sv_attempt) {
-        void *svb = nullptr;
-        if ((st = ctx_scratch(ctx, 9, sizeof(uint64_t) * (size_t)sv_cap, &svb)) != DELTA_OK) return st;
-        rc.sv = (uint64_t *)svb;
-        rc.sv_cap = sv_cap;
-        if ((e = cudaMemsetAsync(queue, 0, 3 * sizeof(unsigned long long), s)) != cudaSuccess)
-          return cuda_error(e, "memset");
-        if ((e = launch_cull(s, m, pa, pb, n_pairs, rc, dstats, ctx->cull_blocks_per_sm)) != cudaSuccess)
-          return cuda_error(e, "cull kernel");
-        ctx->launches += 1;
-        if ((e = cudaMemcpyAsync(&hsv, sv_count, sizeof(hsv), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(s)) != cudaSuccess)
-          return cuda_error(e, "survivor count");
-        if ((int64_t)hsv <= sv_cap) break;
-        sv_cap = (int64_t)hsv + hsv / 4;
-      }
-      if ((e = launch_survivors(driver, s, m, pa, pb, rc, dstats, (int64_t)hsv, ctx->surv_blocks_per_sm)) !=
-          cudaSuccess)
-        return cuda_error(e, "survivor kernel");
-      k_sv_evaluated<<<1, 1, 0, s>>>(sv_count, rc.sv_cap, dstats, nullptr);
-      ctx->launches += 2;
-      e = cudaGetLastError();
-    } else {
-      e = precision == DELTA_F32
-            ? launch_detect_prec<float>(driver, s, m, pa, pb, row_offset, n_pairs, total_rows, rc, dstats, queue)
-            : launch_detect_prec<xf64>(driver, s, m, pa, pb, row_offset, n_pairs, total_rows, rc, dstats, queue);
-      ctx->launches += 1;
-    }
+    if ((st = raw_contacts(ctx, cap, rc)) != DELTA_OK) return st;
+    if (attempt > 0 && (e = cudaMemsetAsync(dev, 0, sizeof(DetectSmall), s)) != cudaSuccess)
+      return cuda_error(e, "detect memset");
+    e = precision == DELTA_F32
+          ? launch_detect_prec<float>(driver, s, m, pa, pb, row_offset, n_pairs, total_rows, rc, &dev->stats, &dev->queue)
+          : launch_detect_prec<xf64>(driver, s, m, pa, pb, row_offset, n_pairs, total_rows, rc, &dev->stats, &dev->queue);
+    ctx->launches += 1;
     if (e != cudaSuccess) return cuda_error(e, "detect kernel");
-    if ((e = cudaMemcpyAsync(&hcount, count, sizeof(hcount), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+    if ((e = cudaMemcpyAsync(host, dev, sizeof(DetectSmall), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
       return cuda_error(e, "detect count");
-    if ((int64_t)hcount <= cap) break;
-    cap = (int64_t)hcount + hcount / 4;
+    if ((int64_t)host->count <= cap) break;
+    cap = (int64_t)host->count + host->count / 4;
   }
-  if (stats || counters) {
-    DevStats h;
-    if ((e = cudaMemcpy(&h, dstats, sizeof h, cudaMemcpyDeviceToHost)) != cudaSuccess)
-      return cuda_error(e, "stats");
-    if (counters) {
-      counters[0] += (int64_t)h.tri_pairs;
-      counters[1] += (int64_t)h.evaluated;
-    }
+  return DELTA_OK;
+}
+
+// bf() (DELTA_DRV_BF in FP64) from delta_detect, cull_bf set, takes the culled drivers' path
+// with FP64 bfSolver on the survivors.  Its contacts are those of the plain path for any
+// meshes: the parameters bfSolver returns lie in [0, 1] (each is clamped or a quotient of
+// numbers in that order), so P and Q lie on the triangles up to the rounding of a few
+// operations on their coordinates, and a pair whose boxes are more than epsA + epsB apart,
+// with 1e-14 of the largest coordinate for that rounding, cannot come within epsA + epsB.
+// (A feature with a NaN vertex has a NaN distance and is never chosen; the boxes hold the
+// other vertices.)  256 bodies of 80 triangles: a call 468 us with the plain kernel, which is
+// FP64-bound, 81 with the culling, its launches and two waits for the host.
+//
+// Scratch slots used here: 2 rows/row_offset, 3 raw contacts, 4 sort temp, 5 small state, 6
+// sort buffers, 9 survivors, 23 body boxes.
+delta_status detect_run(delta_ctx *ctx, int driver, int precision, const delta_meshes &m, const int32_t *pa,
+                        const int32_t *pb, int64_t n_pairs, const delta_contacts *out, int64_t *n_out,
+                        delta_stats *stats, int64_t *counters, const Pose *pose, bool cull_bf) {
+  cudaStream_t s = ctx->stream;
+  delta_status st;
+  cudaError_t e;
+  void *small = nullptr, *pin = nullptr;
+  if ((st = ctx_scratch(ctx, 5, sizeof(DetectSmall), &small)) != DELTA_OK) return st;
+  if ((st = ctx_pinned(ctx, sizeof(DetectSmall), &pin)) != DELTA_OK) return st;
+  DetectSmall *dev = (DetectSmall *)small, *host = (DetectSmall *)pin;
+  // raw contact buffer: at least the caller's capacity; grown and rerun when it overflows
+  const int64_t cap = out->capacity > 1024 ? out->capacity : 1024;
+  RawContacts rc{};
+  rc.tbits = 16;
+  const bool culled_bf = cull_bf && driver == DELTA_DRV_BF && precision == DELTA_F64;
+  if (culled_bf) rc.rel_slack = 1e-14;
+  if (culled_bf || driver == DELTA_DRV_BF_CERT || driver == DELTA_DRV_BF_CULLED || driver == DELTA_DRV_LEARNED)
+    st = detect_culled(ctx, culled_bf ? (int)DELTA_DRV_BF_CULLED : driver, m, pa, pb, n_pairs, cap, dev, host, pose, rc);
+  else
+    st = detect_rows(ctx, driver, precision, m, pa, pb, n_pairs, cap, dev, host, rc);
+  if (st != DELTA_OK) return st;
+  const DevStats h = host->stats;
+  if (counters) {
+    counters[0] += (int64_t)h.tri_pairs;
+    counters[1] += (int64_t)h.evaluated;
   }
   if (stats) {
-    DevStats h;
-    if ((e = cudaMemcpy(&h, dstats, sizeof h, cudaMemcpyDeviceToHost)) != cudaSuccess)
-      return cuda_error(e, "stats");
     for (int i = 0; i < 17; ++i) stats->newton_hist[i] = (int64_t)h.hist[i];
     stats->penalty_fails = (int64_t)h.penalty_fails;
     stats->batch_fails = (int64_t)h.batch_fails;
     stats->batch_size = (int64_t)h.batch_size;
     stats->batch_error = h.batch_error;
   }
-  const int64_t n = (int64_t)hcount;
+  const int64_t n = (int64_t)host->count;
   *n_out = n;
   if (n == 0) return DELTA_OK;
   // sort (key, index) and gather into the caller's arrays
   int64_t *perm_in = nullptr;
-  void *sbuf = nullptr;
+  void *sbuf = nullptr, *temp = nullptr;
   if ((st = ctx_scratch(ctx, 6, sizeof(int64_t) * 2 * (size_t)n + sizeof(uint64_t) * (size_t)n, &sbuf)) != DELTA_OK)
     return st;
   perm_in = (int64_t *)sbuf;
@@ -1111,7 +1153,7 @@ delta_status detect_run(delta_ctx *ctx, int driver, int precision, const delta_m
   ctx->launches += 1;
   int end_bit = 33;
   while (end_bit < 64 && ((int64_t)1 << (end_bit - 32)) < n_pairs) ++end_bit;
-  temp_bytes = 0;
+  size_t temp_bytes = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, rc.key, key_out, perm_in, perm_out, n, 0, end_bit, s);
   if ((st = ctx_scratch(ctx, 4, temp_bytes, &temp)) != DELTA_OK) return st;
   if ((e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, rc.key, key_out, perm_in, perm_out, n, 0, end_bit, s)) !=

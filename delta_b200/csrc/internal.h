@@ -57,10 +57,12 @@ struct Pose;  // pose.cuh
 // Particle-pair drivers (detect.cu).  `pose`: for the certified driver, the bodies' poses
 // from which the current vertices and the body boxes are formed (the meshes' vertex arrays
 // need not be current), or null (then the meshes' vertices are read and the body boxes
-// computed from them).
+// computed from them).  `cull_bf`: DELTA_DRV_BF in FP64 through the box culling (the same
+// contacts); false keeps every triangle pair's bfSolver (the simulation's plain driver).
 delta_status detect_run(delta_ctx *ctx, int driver, int precision, const delta_meshes &m, const int32_t *pa,
                         const int32_t *pb, int64_t n_pairs, const delta_contacts *out, int64_t *n_out,
-                        delta_stats *stats, int64_t *counters = nullptr, const Pose *pose = nullptr);
+                        delta_stats *stats, int64_t *counters = nullptr, const Pose *pose = nullptr,
+                        bool cull_bf = false);
 
 // Resident blocks per SM of a culled driver's two kernels (the culling kernel and the
 // survivors' solver): the largest caps delta_ctx::cull_blocks_per_sm / surv_blocks_per_sm

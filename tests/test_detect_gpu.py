@@ -159,3 +159,36 @@ def test_empty_pair_list(ctx):
     m = Meshes.from_bodies(bodies, eps_b, fric, ids)
     out, _ = detect(ctx, 0, m, [], [])
     assert out.count == 0
+
+
+@pytest.mark.parametrize("kind", ["plain", "far", "collapsed", "nan", "inf", "touching", "wide"])
+def test_bf_driver_leaves_out_no_contact(ctx, oracle, kind):
+    """delta_detect's bf() tests boxes before it solves: the contacts stay the serial loop's,
+    bit for bit, far from the origin, with collapsed triangles, with vertices that are not
+    numbers, at distance zero with no margin, and with a margin wider than the bodies."""
+    from delta_b200.detection import DRV_BF, Meshes, detect
+
+    bodies, pa, pb, eps_b, fric, ids = _scene(11, sizes=(20, 40, 80, 20))
+    rng = np.random.default_rng(7)
+    if kind == "far":
+        bodies = [b + np.array([[3e6], [-7e6], [1e7]]) for b in bodies]
+    elif kind == "collapsed":
+        for b in bodies:
+            t = b.reshape(3, -1, 3)
+            t[:, 0, :] = t[:, 0, :1]  # a point
+            t[:, 1, 2] = t[:, 1, 1]  # a segment
+    elif kind in ("nan", "inf"):
+        for b in bodies:
+            b[rng.integers(0, 3, 6), rng.integers(0, b.shape[1], 6)] = np.nan if kind == "nan" else np.inf
+    elif kind == "touching":
+        bodies = [bodies[0], bodies[0].copy(), bodies[0] + 0.25, bodies[0] + 0.25]
+        eps_b = np.zeros(4)
+    elif kind == "wide":
+        eps_b = np.full(4, 0.2)
+    m = Meshes.from_bodies(bodies, eps_b, fric, ids)
+    g = detect(ctx, DRV_BF, m, pa, pb)[0].to_numpy()
+    o, _, _ = _oracle_contacts(oracle, DRV_BF, bodies, pa, pb, eps_b, fric, ids)
+    assert len(g) == len(o)
+    assert len(g) > 0
+    for f in FIELDS:
+        assert np.array_equal(g[f], o[f], equal_nan=True), f
