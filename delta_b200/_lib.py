@@ -71,6 +71,8 @@ SIGNATURES: dict[str, tuple[list, object]] = {
     "delta_mlp_act_grad": ([vp, i64, C.c_int, vp, vp, vp], C.c_int),
     "delta_mlp_colsum": ([vp, i64, C.c_int, vp, vp], C.c_int),
     "delta_adam": ([vp, i64, vp, vp, vp, vp, C.c_float, C.c_float, C.c_float, C.c_float, i64, vp], C.c_int),
+    "delta_mlp_train_step": ([vp, i64, vp, vp, vp, C.c_float, vp, vp, vp, vp, vp, C.c_float, C.c_float, C.c_float,
+                              C.c_float, i64, vp], C.c_int),
     "delta_to_bf16": ([vp, i64, vp, vp], C.c_int),
     "delta_penalty_warm": ([vp, i64, vp, vp, i64, vp, f8, vp, vp, vp, vp], C.c_int),
     "delta_learned_refine": ([vp, i64, vp, vp, i64, vp, i32, i32, f8, vp, vp, vp, vp], C.c_int),

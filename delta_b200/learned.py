@@ -76,6 +76,7 @@ class WarmStartMLP:
         self.grads = torch.zeros_like(self.params)
         self.m = torch.zeros_like(self.params)
         self.v = torch.zeros_like(self.params)
+        self.loss = torch.zeros(1, dtype=torch.float32, device=self.dev)
         self.steps = 0
         self._ws_rows = 0
         self._refresh_bf16()
@@ -127,7 +128,6 @@ class WarmStartMLP:
         self.dY = torch.empty((M, OUT), **b16)
         self.dH = torch.empty((M, HIDDEN), **f32)
         self.dZ = torch.empty((M, HIDDEN), **b16)
-        self.loss = torch.zeros(1, **f32)
         self._ws_rows = M
 
     # -- kernels -----------------------------------------------------------------------
@@ -192,6 +192,17 @@ class WarmStartMLP:
                                self.params_bf16.data_ptr()))
 
     def train_step(self, X, T, valid, n_valid: int, lr=1e-3):
+        """forward, backward and adam.  On the tcgen05 engine one fused call
+        (delta_mlp_train_step), which leaves the forward workspaces (Z, H, Y) alone."""
+        M = X.shape[0]
+        if M > 0 and getattr(self.ctx, "mlp_engine", "tcgen05") == "tcgen05" and not (X.data_ptr() | T.data_ptr()) & 15:
+            self.steps += 1
+            check(lib().delta_mlp_train_step(self.ctx.handle, M, X.data_ptr(), T.data_ptr(), valid.data_ptr(),
+                                             1.0 / max(n_valid, 1), self.params.data_ptr(),
+                                             self.params_bf16.data_ptr(), self.grads.data_ptr(), self.m.data_ptr(),
+                                             self.v.data_ptr(), lr, 0.9, 0.999, 1e-8, self.steps,
+                                             self.loss.data_ptr()))
+            return
         self.forward(X)
         self.backward(X, T, valid, n_valid)
         self.adam(lr)

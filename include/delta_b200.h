@@ -554,6 +554,15 @@ delta_status delta_mlp_colsum(delta_ctx *ctx, int64_t M, int N, const void *dZ_b
  * w_bf16 (optional) receives the BF16 copy. */
 delta_status delta_adam(delta_ctx *ctx, int64_t n, float *w, const float *g, float *m, float *v, float lr, float b1,
                         float b2, float eps, int64_t step, void *w_bf16);
+/* One training step of the network (tcgen05 engine only): forward, the MSE over valid rows
+ * (inv_n = 1 / their number), gradients g (overwritten), loss[1] (overwritten) and Adam on
+ * the FP32 weights w with moments m, v; w_bf16 is read as the layers' weights and refreshed.
+ * X rows of 32 BF16, T rows of 4 FP32; X, T and w_bf16 16-byte aligned; M > 0.  The same
+ * roundings as delta_gemm_bf16 / delta_mlp_bias_act / _mse / _act_grad / _colsum /
+ * delta_adam in turn, sums over the batch in another (fixed) order. */
+delta_status delta_mlp_train_step(delta_ctx *ctx, int64_t M, const void *X_bf16, const float *T,
+                                  const uint8_t *valid, float inv_n, float *w, void *w_bf16, float *g, float *m,
+                                  float *v, float lr, float b1, float b2, float eps, int64_t step, float *loss);
 delta_status delta_to_bf16(delta_ctx *ctx, int64_t n, const float *x, void *y_bf16);
 /* penaltySolver(..., maxError, int& iterations) (penalty.cpp:434-582, FP64 reference
  * arithmetic) started from x0 [n][4] instead of 0.33 (x0 NULL: 0.33).  iterations [n]
