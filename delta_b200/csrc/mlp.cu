@@ -465,66 +465,75 @@ __global__ void __launch_bounds__(32 * kInferWarps, 2)
 }
 
 // ---------------------------------------------------------------------------------------
-// fused inference on the 5th-generation tensor cores (tcgen05, accumulators in TMEM).
-// One CTA = 8 warps = 256 threads works on tiles of 128 pairs: pair r of the tile is row r
-// of every layer's M=128 MMA and TMEM lane r of its accumulator; warps w and w+4 both read
-// lanes 32(w%4)..32(w%4)+31 (the TMEM lanes a warp may access), w < 4 columns 0..63 and
-// w >= 4 columns 64..127.  Two CTAs fit on an SM, so one's MMAs overlap the other's
-// epilogue.
+// fused inference on the 5th-generation tensor cores (tcgen05, accumulators in TMEM), from
+// the pair list to x0.  One CTA of 512 threads per SM: its four warpgroups share the weights
+// in shared memory and work on tiles of 128 pairs of their own, so that the MMAs, barriers
+// and loads of one tile are hidden behind the GELU epilogues of three others (bound: the
+// tanh of the XU pipe, 384 a pair).  Pair r of a tile is thread r of the warpgroup, which
+// forms its features in FP64 (k_canon's arithmetic), row r of every layer's M=128 MMA and
+// TMEM lane r of its accumulator (128 columns a warpgroup).
 // Operands live in shared memory in the canonical K-major layout without swizzle:
 // element (r, k) of a [rows][K] BF16 matrix sits at (r/8)*SBO + (k/8)*128 + (r%8)*16 +
 // (k%8)*2 bytes (8x8 core matrices of 128 bytes; LBO = 128 between K neighbours, SBO =
-// 16*K between row groups).  One thread issues the MMAs of a layer (K/16 of them,
-// 128x128x16 or 128x16x16), commits them to an mbarrier, and every thread then reads its
-// row of the accumulator with tcgen05.ld, adds the bias, applies GELU and writes the BF16
-// row back as the next layer's A operand.  Waits on the mbarrier are bounded: on time-out
-// the kernel records it in *err, stops, and frees its TMEM.
+// 16*K between row groups).  One thread of the warpgroup issues the MMAs of a layer (K/16 of
+// them, 128x128x16 or 128x16x16), commits them to the warpgroup's mbarrier, and every thread
+// then reads its row of the accumulator with tcgen05.ld, adds the bias, applies GELU and
+// writes the BF16 row back as the next layer's A operand.  Waits on the mbarrier are
+// bounded: on time-out the warpgroup records it in *err and stops; the TMEM is freed when
+// all four are done.
+// 1,000,003 pairs: 256 us before (features 47 by a kernel of their own, then two CTAs of
+// one tile each per SM, 209), 184 now.  Slower: all 128 threads polling the mbarrier (195), the
+// next tile's features formed while the last layer runs (194).
 // ---------------------------------------------------------------------------------------
+constexpr int kTcGroups = 4, kTcThreads = kTcGroups * kTcRows;
+
 struct TcSmem {
-  __nv_bfloat16 w1[kHid * kIn];         // 8 KB   (N=128, K=32)
+  __nv_bfloat16 w1[kHid * kIn];        // 8 KB   (N=128, K=32)
   __nv_bfloat16 w2[kHid * kHid];        // 32 KB  (N=128, K=128)
   __nv_bfloat16 w3[kHid * kHid];        // 32 KB
   __nv_bfloat16 w4[kTcW4Rows * kHid];   // 4 KB   (N=16, K=128; rows 4..15 zero)
-  __nv_bfloat16 ah[kTcRows * kHid];     // 32 KB  A operand: layer-1 input (K=32) or hidden (K=128)
+  __nv_bfloat16 ah[kTcGroups][kTcRows * kHid];  // 32 KB each: A operand, layer-1 input (K=32) or hidden (K=128)
   float bias[3 * kHid + kTcW4Rows];
-  uint64_t mbar;
+  uint64_t mbar[kTcGroups];
   uint32_t tmem_base;
-  int abort;
+  int abort[kTcGroups];
 };
 
-// one layer: the elected thread issues K/16 MMAs into TMEM and commits; everyone waits
-// (at most `spin` polls).  Returns false (and sets the CTA's abort flag) when the wait
-// timed out.  `withhold` (the time-out test only) issues neither the MMAs nor the commit,
-// so the barrier never completes and the wait runs out with nothing in flight.
-__device__ __forceinline__ bool tc_layer(TcSmem &sm, const __nv_bfloat16 *A, const __nv_bfloat16 *W, int K, int N,
-                                         uint32_t &phase, uint32_t spin = kTcSpin, bool withhold = false) {
+// barrier of the calling warpgroup's 128 threads
+__device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory"); }
+
+// one layer of warpgroup g: its first thread issues K/16 MMAs into TMEM and commits;
+// everyone waits (at most `spin` polls).  Returns false (and sets the warpgroup's abort
+// flag) when the wait timed out.  `withhold` (the time-out test only) issues neither the
+// MMAs nor the commit, so the barrier never completes and the wait runs out with nothing in
+// flight.
+__device__ __forceinline__ bool tc_layer(TcSmem &sm, int g, uint32_t tmem, const __nv_bfloat16 *W, int K, int N,
+                                         uint32_t &phase, uint32_t spin, bool withhold = false) {
   // make the generic-proxy stores of A visible to the tensor cores, then synchronise
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  group_sync(g);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (threadIdx.x == 0) {
-    const uint32_t a0 = (uint32_t)__cvta_generic_to_shared(A), w0 = (uint32_t)__cvta_generic_to_shared(W);
+  if ((threadIdx.x & (kTcRows - 1)) == 0) {
+    const uint32_t a0 = (uint32_t)__cvta_generic_to_shared(sm.ah[g]), w0 = (uint32_t)__cvta_generic_to_shared(W);
     const uint32_t idesc = tc_idesc(kTcRows, N);
     if (!withhold) {
       for (int s = 0; s < K / 16; ++s)
-        tc_mma(sm.tmem_base, tc_desc(a0 + 256u * s, 16u * K), tc_desc(w0 + 256u * s, 16u * K), idesc, s > 0 ? 1u : 0u);
-      tc_commit(&sm.mbar);
+        tc_mma(tmem, tc_desc(a0 + 256u * s, 16u * K), tc_desc(w0 + 256u * s, 16u * K), idesc, s > 0 ? 1u : 0u);
+      tc_commit(&sm.mbar[g]);
     }
-    if (!tc_wait(&sm.mbar, phase, spin)) sm.abort = 1;
+    if (!tc_wait(&sm.mbar[g], phase, spin)) sm.abort[g] = 1;
   }
-  __syncthreads();
+  group_sync(g);
   phase ^= 1u;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  return sm.abort == 0;
+  return sm.abort[g] == 0;
 }
 
-constexpr int kTcThreads = 2 * kTcRows;
-
-__global__ void __launch_bounds__(kTcThreads, 2)
-    k_mlp_infer_tc(int64_t n, const __nv_bfloat16 *__restrict__ feat, const float *__restrict__ params,
-                   const __nv_bfloat16 *__restrict__ wb, float *__restrict__ x0, int *__restrict__ err,
-                   uint32_t spin, int withhold) {
+__global__ void __launch_bounds__(kTcThreads, 1)
+    k_mlp_infer_tc(int64_t n, const double *__restrict__ a, const double *__restrict__ b, int64_t ld,
+                   const float *__restrict__ params, const __nv_bfloat16 *__restrict__ wb, float *__restrict__ x0,
+                   int *__restrict__ err, uint32_t spin, int withhold) {
   extern __shared__ __align__(128) unsigned char tc_smem_raw[];
   TcSmem &sm = *reinterpret_cast<TcSmem *>(tc_smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -538,78 +547,92 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     sm.bias[2 * kHid + e] = params[kOffB3 + e];
   }
   if (tid < kTcW4Rows) sm.bias[3 * kHid + tid] = tid < kOut ? params[kOffB4 + tid] : 0.f;
-  if (tid == 0) {
-    sm.abort = 0;
-    const unsigned a = (unsigned)__cvta_generic_to_shared(&sm.mbar);
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(a) : "memory");
+  if (tid < kTcGroups) {
+    sm.abort[tid] = 0;
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&sm.mbar[tid]))
+                 : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  constexpr uint32_t kCols = kTcGroups * kTmemCols;
   if (warp == 0) {
     const unsigned dst = (unsigned)__cvta_generic_to_shared(&sm.tmem_base);
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(kTmemCols)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(kCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const int r = tid & (kTcRows - 1), half = tid >> 7;  // row of the tile, column half
+  const int r = tid & (kTcRows - 1), g = tid >> 7;  // row of the tile, warpgroup
+  const uint32_t tmem = sm.tmem_base + g * kTmemCols;
   // this thread's TMEM lane (row) in bits 16..31 of the address, column in bits 0..15
-  const uint32_t tlane = sm.tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+  const uint32_t tlane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+  char *ah = reinterpret_cast<char *>(sm.ah[g]);
   uint32_t phase = 0;
+  bool ok = true;
   const int64_t tiles = (n + kTcRows - 1) / kTcRows;
-  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+  // (the warpgroups of one SM take tiles a grid apart: short lists spread over the SMs)
+  for (int64_t tile = blockIdx.x + (int64_t)g * gridDim.x; tile < tiles; tile += (int64_t)kTcGroups * gridDim.x) {
     const int64_t row = tile * kTcRows + r;
-    // layer-1 input: two of the row's four 16-byte feature chunks per thread
     {
-      const uint4 *src = reinterpret_cast<const uint4 *>(feat + 32 * (row < n ? row : n - 1));
+      xf64 A[3][3], B[3][3];
+      float f[18];
+      bool fine;
+      canon_pair(a, b, ld, row < n ? row : n - 1, A, B, f, fine);
+      uint32_t w[16];
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int kc = 2 * half + q;
-        *reinterpret_cast<uint4 *>(reinterpret_cast<char *>(sm.ah) + tc_chunk(r, kc, kIn)) = __ldg(src + kc);
-      }
+      for (int k = 0; k < 9; ++k) w[k] = pack_bf16(f[2 * k], f[2 * k + 1]);
+#pragma unroll
+      for (int k = 9; k < 16; ++k) w[k] = 0u;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        *reinterpret_cast<uint4 *>(ah + tc_chunk(r, k, kIn)) =
+            make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
     }
     int K = kIn;
-    const __nv_bfloat16 *Ws[3] = {sm.w1, sm.w2, sm.w3};
-    bool ok = true;
     for (int l = 0; l < 3; ++l) {
-      ok = tc_layer(sm, sm.ah, Ws[l], K, kHid, phase, spin, withhold != 0 && l == 0);
+      ok = tc_layer(sm, g, tmem, l == 0 ? sm.w1 : l == 1 ? sm.w2 : sm.w3, K, kHid, phase, spin, withhold != 0 && l == 0);
       if (!ok) break;
-      // bias + GELU of this thread's 64 columns of its row, into the hidden A tile
+      // bias + GELU of this thread's row, into the hidden A tile
 #pragma unroll 1
-      for (int c = 64 * half; c < 64 * half + 64; c += 32) {
+      for (int c = 0; c < kHid; c += 32) {
         float v[32];
         tc_ld32(tlane + (uint32_t)c, v);
         uint32_t w[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k)
-          w[k] = pack_bf16(gelu(v[2 * k] + sm.bias[l * kHid + c + 2 * k]),
-                           gelu(v[2 * k + 1] + sm.bias[l * kHid + c + 2 * k + 1]));
-        char *dst = reinterpret_cast<char *>(sm.ah);
+          w[k] = pack_bf16(gelu2(__fadd2_rn(make_float2(v[2 * k], v[2 * k + 1]),
+                                            *reinterpret_cast<const float2 *>(sm.bias + l * kHid + c + 2 * k))));
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<uint4 *>(dst + tc_chunk(r, c / 8 + q, kHid)) =
+          *reinterpret_cast<uint4 *>(ah + tc_chunk(r, c / 8 + q, kHid)) =
               make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
       }
       K = kHid;
     }
     if (!ok) break;
-    if (!tc_layer(sm, sm.ah, sm.w4, kHid, kTcW4Rows, phase, spin)) break;
-    if (half == 0) {
-      float v[16];
-      tc_ld16(tlane, v);
-      if (row < n)
-        *reinterpret_cast<float4 *>(x0 + 4 * row) =
-            make_float4(v[0] + sm.bias[3 * kHid], v[1] + sm.bias[3 * kHid + 1], v[2] + sm.bias[3 * kHid + 2],
-                        v[3] + sm.bias[3 * kHid + 3]);
-    }
+    if (!(ok = tc_layer(sm, g, tmem, sm.w4, kHid, kTcW4Rows, phase, spin))) break;
+    float v[16];
+    tc_ld16(tlane, v);
+    if (row < n)
+      *reinterpret_cast<float4 *>(x0 + 4 * row) =
+          make_float4(v[0] + sm.bias[3 * kHid], v[1] + sm.bias[3 * kHid + 1], v[2] + sm.bias[3 * kHid + 2],
+                      v[3] + sm.bias[3 * kHid + 3]);
   }
-  if (sm.abort && tid == 0) atomicExch(err, 1);
+  if (!ok && r == 0) {
+    // after a time-out: whatever was issued must end before the TMEM is freed (bounded)
+    if (!withhold) {
+      tc_commit(&sm.mbar[g]);
+      tc_wait(&sm.mbar[g], phase, spin);
+    }
+    atomicExch(err, 1);
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sm.tmem_base), "r"(kTmemCols)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sm.tmem_base), "r"(kCols)
                  : "memory");
   }
 }
@@ -1174,19 +1197,13 @@ __global__ void __launch_bounds__(128, 8) k_learned_refine(int64_t n, const doub
 
 inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t > 0 ? (n + t - 1) / t : 1); }
 
-// Features into scratch, then the network on `engine`; with the tcgen05 engine *err_out
+// The network on `engine` (mma.sync: on features written to scratch first); with the tcgen05 engine *err_out
 // receives the device time-out flag (zeroed here, set by the kernel).
 delta_status mlp_infer_launch(delta_ctx *ctx, int engine, int64_t n, const double *a, const double *b, int64_t ld,
                               const float *params, const void *params_bf16, float *x0, int **err_out,
                               uint32_t spin = kTcSpin, int withhold = 0) {
-  void *fbuf;
-  delta_status st = ctx_scratch(ctx, 15, sizeof(__nv_bfloat16) * 32 * (size_t)n, &fbuf);
-  if (st != DELTA_OK) return st;
-  __nv_bfloat16 *feat = static_cast<__nv_bfloat16 *>(fbuf);
-  k_canon<<<nblk(n), 256, 0, ctx->stream>>>(n, a, b, ld, nullptr, nullptr, feat, nullptr, nullptr);
-  ctx->launches += 1;
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_error(e, "mlp features");
+  delta_status st;
+  cudaError_t e;
   const __nv_bfloat16 *wb = static_cast<const __nv_bfloat16 *>(params_bf16);
   if (engine == DELTA_MLP_TCGEN05) {
     void *ebuf;
@@ -1200,10 +1217,16 @@ delta_status mlp_infer_launch(delta_ctx *ctx, int engine, int64_t n, const doubl
       configured_device = ctx->device;
     }
     const int64_t tiles = (n + kTcRows - 1) / kTcRows;
-    const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * kNumSMs);
-    k_mlp_infer_tc<<<grid, kTcThreads, sizeof(TcSmem), ctx->stream>>>(n, feat, params, wb, x0, err, spin, withhold);
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, kNumSMs);
+    k_mlp_infer_tc<<<grid, kTcThreads, sizeof(TcSmem), ctx->stream>>>(n, a, b, ld, params, wb, x0, err, spin, withhold);
     if (err_out) *err_out = err;
   } else {
+    void *fbuf;
+    if ((st = ctx_scratch(ctx, 15, sizeof(__nv_bfloat16) * 32 * (size_t)n, &fbuf)) != DELTA_OK) return st;
+    __nv_bfloat16 *feat = static_cast<__nv_bfloat16 *>(fbuf);
+    k_canon<<<nblk(n), 256, 0, ctx->stream>>>(n, a, b, ld, nullptr, nullptr, feat, nullptr, nullptr);
+    ctx->launches += 1;
+    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "mlp features");
     static thread_local int configured_device = -1;
     if (configured_device != ctx->device) {
       e = cudaFuncSetAttribute(k_mlp_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(InferSmem));

@@ -34,6 +34,27 @@ __device__ __forceinline__ float gelu_grad(float x) {
   return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * kGeluK * fmaf(3.f * kGeluC, x2, 1.f);
 }
 
+// gelu and gelu_grad of two values with the packed FP32 operations of sm_100 (one issue slot
+// for both; each lane rounds as the scalar operation does: gelu2 is gelu bit for bit, and gelu_grad2 spells
+// out the multiply-adds that the compiler forms in gelu_grad).
+// The tcgen05 kernels' epilogues are bound by issue slots and the tanh unit.
+__device__ __forceinline__ float2 splat2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 gelu2(float2 x) {
+  const float2 u = __fmul2_rn(x, __ffma2_rn(splat2(kGeluC * kGeluK), __fmul2_rn(x, x), splat2(kGeluK)));
+  const float2 h = __fmul2_rn(splat2(0.5f), x);
+  return __ffma2_rn(h, make_float2(tanh_hw(u.x), tanh_hw(u.y)), h);
+}
+__device__ __forceinline__ float2 gelu_grad2(float2 x) {
+  const float2 x2 = __fmul2_rn(x, x);
+  const float2 u = __fmul2_rn(x, __ffma2_rn(splat2(kGeluC * kGeluK), x2, splat2(kGeluK)));
+  const float2 th = make_float2(tanh_hw(u.x), tanh_hw(u.y));
+  const float2 sech2 = __ffma2_rn(make_float2(-th.x, -th.y), th, splat2(1.f));
+  const float2 p = __fmul2_rn(__fmul2_rn(__fmul2_rn(splat2(0.5f), x), sech2), splat2(kGeluK));
+  const float2 q = __fmul2_rn(p, __ffma2_rn(splat2(3.f * kGeluC), x2, splat2(1.f)));
+  return __ffma2_rn(splat2(0.5f), __fadd2_rn(splat2(1.f), th), q);
+}
+__device__ __forceinline__ uint32_t pack_bf16(float2 v) { return pack_bf16(v.x, v.y); }
+
 // Adam (Kingma & Ba 2015) on FP32 master weight i with gradient gi; refreshes the BF16 copy.
 __device__ __forceinline__ void adam_update(int64_t i, float gi, float *w, float *m, float *v, float lr, float b1,
                                             float b2, float eps, float c1, float c2, __nv_bfloat16 *wb) {
