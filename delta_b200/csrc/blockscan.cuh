@@ -12,39 +12,61 @@
 namespace delta {
 
 constexpr int kBlockScanThreads = 1024, kBlockScanItems = 8;
-// one tile: a CTA that loops over two or more tiles was slower than cub's two kernels (the
-// hopper's 10,001-entry slave lists: 8% of its replayed step)
-constexpr int64_t kBlockScanMax = (int64_t)kBlockScanThreads * kBlockScanItems;
+// Up to four tiles of 8,192 entries.  (With a run of 8 entries per thread, whose 64-byte
+// strides cost the CTA's loads and stores 8 sectors a request, one full tile took 7 us of a
+// hopper step and two were slower than cub's two kernels, 5 us for 10,001 entries.)
+constexpr int64_t kBlockScanMax = 4 * (int64_t)kBlockScanThreads * kBlockScanItems;
 
-// out[i] = in[0] + ... + in[i-1] over tiles of 8192 entries, the running total carried
-// from tile to tile (integer sums: exact in any order).
+// out[i] = in[0] + ... + in[i-1] (integer sums: exact in any order).  A warp takes 256
+// consecutive entries of a tile in 8 rounds of 32, so that its loads and stores are whole
+// lines; the rounds' scans run side by side, the warps' totals are scanned by the first
+// warp, and the running total is carried from tile to tile.
 template <class T>
 __global__ void __launch_bounds__(kBlockScanThreads) k_block_exclusive_scan(const T *__restrict__ in,
                                                                             T *__restrict__ out, int64_t n) {
   dep_sync();
-  using Scan = cub::BlockScan<T, kBlockScanThreads>;
-  __shared__ typename Scan::TempStorage tmp;
-  __shared__ T carry;
+  __shared__ T wsum[kBlockScanThreads / 32], carry;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (threadIdx.x == 0) carry = T(0);
-  __syncthreads();
   for (int64_t base = 0; base < n; base += (int64_t)kBlockScanThreads * kBlockScanItems) {
-    T v[kBlockScanItems];
+    const int64_t i0 = base + (int64_t)w * 32 * kBlockScanItems + lane;
+    T v[kBlockScanItems], own[kBlockScanItems];
+#pragma unroll
+    for (int j = 0; j < kBlockScanItems; ++j) v[j] = own[j] = i0 + 32 * j < n ? in[i0 + 32 * j] : T(0);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+      for (int j = 0; j < kBlockScanItems; ++j) {
+        const T y = __shfl_up_sync(0xffffffffu, v[j], o);
+        if (lane >= o) v[j] += y;
+      }
+    T total = T(0);  // of the rounds before j, then of the warp
 #pragma unroll
     for (int j = 0; j < kBlockScanItems; ++j) {
-      const int64_t i = base + (int64_t)threadIdx.x * kBlockScanItems + j;
-      v[j] = i < n ? in[i] : T(0);
+      const T t = __shfl_sync(0xffffffffu, v[j], 31);
+      v[j] += total - own[j];
+      total += t;
     }
-    T total;
-    Scan(tmp).ExclusiveSum(v, v, total);
-    const T c = carry;
-#pragma unroll
-    for (int j = 0; j < kBlockScanItems; ++j) {
-      const int64_t i = base + (int64_t)threadIdx.x * kBlockScanItems + j;
-      if (i < n) out[i] = v[j] + c;
-    }
-    __syncthreads();  // every thread has read carry and tmp
-    if (threadIdx.x == 0) carry = c + total;
+    if (lane == 0) wsum[w] = total;
     __syncthreads();
+    if (w == 0) {
+      const T s = wsum[lane];
+      T x = s;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const T y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      wsum[lane] = x - s + carry;
+      __syncwarp();
+      if (lane == 31) carry += x;
+    }
+    __syncthreads();
+    const T before = wsum[w];
+#pragma unroll
+    for (int j = 0; j < kBlockScanItems; ++j)
+      if (i0 + 32 * j < n) out[i0 + 32 * j] = v[j] + before;
+    __syncthreads();  // wsum is written again by the next tile
   }
 }
 

@@ -50,7 +50,7 @@ struct RawContacts {
   // fixed-capacity certified driver: contacts counted per pair (pcnt, zeroed by the culling)
   // and each contact's rank of arrival within its pair (slot), for the sort-free ordering;
   // null elsewhere
-  unsigned long long *pcnt;
+  uint32_t *pcnt;
   uint32_t *slot;
   // culled drivers: the body-pair work queue of the culling kernel (zeroed before it runs);
   // null: blocks take the pairs by a fixed stride
@@ -175,7 +175,7 @@ __device__ __forceinline__ void emit(const RawContacts &rc, bool take, const dou
   const int64_t pos = agg_slot(rc.count);
   if (pos < rc.cap) {
     write_contact(rc, pos, pq, r, tb);
-    if (rc.pcnt) rc.slot[pos] = (uint32_t)atomicAdd(rc.pcnt + r.k, 1ull);
+    if (rc.pcnt) rc.slot[pos] = atomicAdd(rc.pcnt + r.k, 1u);
   }
 }
 
@@ -800,28 +800,32 @@ __global__ void k_gather_fixed(RawContacts rc, const int64_t *perm, delta_contac
 
 // Sort-free ordering of the fixed-capacity certified driver's contacts, step 1: contact c
 // of pair k goes to its pair's bucket, at poff[k] + its rank of arrival, with its key.
-__global__ void k_bucket_contacts(RawContacts rc, const int64_t *poff, int64_t *bidx, uint64_t *bkey) {
+__global__ void k_bucket_contacts(RawContacts rc, const uint32_t *poff, int64_t *bidx, uint64_t *bkey) {
   dep_sync();
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned long long cnt = *rc.count;
   const int64_t n = (int64_t)cnt < rc.cap ? (int64_t)cnt : rc.cap;
   if (c >= n) return;
   const uint64_t key = rc.key[c];
-  const int64_t j = poff[(int64_t)(key >> (2 * rc.tbits))] + rc.slot[c];
+  const int64_t j = (int64_t)poff[key >> (2 * rc.tbits)] + rc.slot[c];
   bidx[j] = c;
   bkey[j] = key;
 }
 
-// Step 2, one thread per bucket entry j: its pair k is the last with poff[k] <= j, its
-// rank the number of smaller keys in the pair's bucket (keys within a pair are distinct),
-// and the contact is written at poff[k] + rank, so the output is in (pair, A triangle,
-// B triangle) order, the order of a stable sort of all keys.  Thread 0 publishes the
-// count and flags an overflow.
-__global__ void k_pair_gather(RawContacts rc, const int64_t *poff, const int64_t *bidx, const uint64_t *bkey,
-                              int64_t n_pairs, delta_contacts out, int64_t *n_out, int *ovf, int ovf_code,
-                              int64_t *count_log) {
+// Step 2, one thread per bucket entry j of pair k (its key's): its rank is the number of
+// smaller keys in the pair's bucket (keys within a pair are distinct), and the contact is
+// written at poff[k] + rank, so the output is in (pair, A triangle, B triangle) order, the
+// order of a stable sort of all keys.  Thread 0 publishes the count and flags an overflow.
+// The block's keys and the 128 on either side are staged in shared memory: the ranks of the
+// buckets that lie within read nothing else.  (With a binary search of poff for the pair
+// and the bucket's keys read from memory one after another: 11 us of a hopper or box step.)
+constexpr int kGatherThreads = 256, kGatherHalo = 128;
+__global__ void __launch_bounds__(kGatherThreads)
+    k_pair_gather(RawContacts rc, const uint32_t *poff, const int64_t *bidx, const uint64_t *bkey, int64_t n_pairs,
+                  delta_contacts out, int64_t *n_out, int *ovf, int ovf_code, int64_t *count_log) {
   dep_sync();
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ uint64_t keys[kGatherThreads + 2 * kGatherHalo];
+  const int64_t blk0 = (int64_t)blockIdx.x * kGatherThreads, j = blk0 + threadIdx.x;
   const unsigned long long cnt = *rc.count;
   if (j == 0) {
     const int64_t n = (int64_t)cnt < out.capacity ? (int64_t)cnt : out.capacity;
@@ -829,18 +833,25 @@ __global__ void k_pair_gather(RawContacts rc, const int64_t *poff, const int64_t
     if (count_log) *count_log = n;
     if ((int64_t)cnt > out.capacity) atomicCAS(ovf, 0, ovf_code);
   }
-  if (j >= poff[n_pairs]) return;
-  int64_t lo = 0, hi = n_pairs;  // poff[0] = 0 <= j < poff[n_pairs]
-  while (lo < hi) {
-    const int64_t mid = (lo + hi + 1) >> 1;
-    if (poff[mid] <= j) lo = mid;
-    else hi = mid - 1;
+  const int64_t total = poff[n_pairs], lo = blk0 - kGatherHalo, hi = blk0 + kGatherThreads + kGatherHalo;
+  if (blk0 >= total) return;
+  for (int t = threadIdx.x; t < kGatherThreads + 2 * kGatherHalo; t += kGatherThreads)
+    if (lo + t >= 0 && lo + t < total) keys[t] = bkey[lo + t];
+  __syncthreads();
+  if (j >= total) return;
+  const uint64_t key = keys[threadIdx.x + kGatherHalo];
+  const int64_t k = (int64_t)(key >> (2 * rc.tbits)), base = poff[k], m = poff[k + 1] - base;
+  const int64_t s = bidx[j], cap = rc.cap, oc = out.capacity;
+  int rank = 0;
+  if (base >= lo && base + m <= hi) {
+    const uint64_t *b = keys + (base - lo);
+#pragma unroll 8
+    for (int i = 0; i < (int)m; ++i) rank += b[i] < key ? 1 : 0;
+  } else {
+#pragma unroll 8
+    for (int64_t i = 0; i < m; ++i) rank += bkey[base + i] < key ? 1 : 0;
   }
-  const int64_t base = poff[lo], m = poff[lo + 1] - base;
-  const uint64_t key = bkey[j];
-  int64_t rank = 0;
-  for (int64_t i = 0; i < m; ++i) rank += bkey[base + i] < key ? 1 : 0;
-  const int64_t d = base + rank, s = bidx[j], cap = rc.cap, oc = out.capacity;
+  const int64_t d = base + rank;
   if (d >= oc) return;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -866,9 +877,10 @@ __global__ void k_accumulate(const DevStats *st, int64_t *counters) {
 
 // End of a fixed-capacity certified detection, one thread: the survivors count as
 // evaluated pairs (a survivor-list overflow raises *ovf), then the step's statistics go
-// to the running counters.
+// to the running counters, the state is cleared for the next step (this is its last
+// reader) and, with `end`, the graph step ends (StepEnd).
 __global__ void k_cert_tail(const unsigned long long *sv_count, int64_t sv_cap, DevStats *st, int *ovf,
-                            int64_t *counters, unsigned long long *queue) {
+                            int64_t *counters, unsigned long long *queue, StepEnd end) {
   dep_sync();
   const unsigned long long c = *sv_count;
   st->evaluated += c;
@@ -877,10 +889,11 @@ __global__ void k_cert_tail(const unsigned long long *sv_count, int64_t sv_cap, 
     counters[0] += (int64_t)st->tri_pairs;
     counters[1] += (int64_t)st->evaluated;
   }
-  if (queue) {  // fixed-capacity state: cleared for the next step (the step's last reader)
+  if (queue) {
     queue[0] = queue[1] = queue[2] = 0ull;
     *st = DevStats{};
   }
+  if (end.step) end.run();
 }
 
 __global__ void k_iota(int64_t *v, int64_t n) {
@@ -1206,7 +1219,7 @@ delta_status detect_fixed_init(cudaStream_t s, void *state, int64_t pair_cap, in
 delta_status detect_run_fixed(delta_ctx *ctx, cudaStream_t s, int driver, const delta_meshes &m, const int32_t *pa,
                               const int32_t *pb, int64_t pair_cap, const delta_contacts &out, int64_t *d_ncontacts,
                               int *d_ovf, int ovf_code, int64_t *d_counters, int64_t *d_count_log, void *state,
-                              void *temp, size_t temp_bytes, const Pose *pose, int tri_bits) {
+                              void *temp, size_t temp_bytes, const Pose *pose, int tri_bits, const StepEnd &end) {
   cudaError_t e;
   const int64_t cap = out.capacity;
   char *p = (char *)state;
@@ -1243,25 +1256,26 @@ delta_status detect_run_fixed(delta_ctx *ctx, cudaStream_t s, int driver, const 
   size_t tb = temp_bytes;
   if (culled) {
     // The culling takes body pairs directly (no rows).  The contacts are ordered without a
-    // sort: counted per pair (rows, zeroed by the culling), the counts scanned into pair
+    // sort: counted per pair (32-bit counts in rows, zeroed by the culling), the counts scanned into pair
     // offsets (row_offset), each contact put in its pair's bucket (indices in perm_out,
     // keys in perm_in, whose identity permutation serves only the other driver), and each
     // pair's bucket ranked by key.  The per-pair arrival ranks use the sort's key_out.
-    rc.pcnt = (unsigned long long *)rows;
+    rc.pcnt = (uint32_t *)rows;
+    uint32_t *poff = (uint32_t *)row_offset;
     rc.slot = (uint32_t *)key_out;
     // programmatic dependent launches (pdl.cuh)
     e = launch_cull(s, m, pa, pb, pair_cap, rc, dstats, ctx->cull_blocks_per_sm, true);
     if (e != cudaSuccess) return cuda_error(e, "cull kernel");
     if ((e = launch_survivors(driver, s, m, pa, pb, rc, dstats, -1, ctx->surv_blocks_per_sm, true)) != cudaSuccess)
       return cuda_error(e, "survivor kernel");
-    if ((e = exclusive_sum(temp, tb, rows, row_offset, pair_cap + 1, s, true)) != cudaSuccess)
+    if ((e = exclusive_sum(temp, tb, rc.pcnt, poff, pair_cap + 1, s, true)) != cudaSuccess)
       return cuda_error(e, "pair contact scan");
     const unsigned cb = (unsigned)((cap + 255) / 256);
-    if ((e = launch_dep(true, k_bucket_contacts, cb, 256, 0, s, rc, row_offset, perm_out, (uint64_t *)perm_in)) !=
+    if ((e = launch_dep(true, k_bucket_contacts, cb, 256, 0, s, rc, poff, perm_out, (uint64_t *)perm_in)) !=
             cudaSuccess ||
-        (e = launch_dep(true, k_pair_gather, cb, 256, 0, s, rc, row_offset, perm_out, (const uint64_t *)perm_in,
+        (e = launch_dep(true, k_pair_gather, cb, kGatherThreads, 0, s, rc, poff, perm_out, (const uint64_t *)perm_in,
                         pair_cap, out, d_ncontacts, d_ovf, ovf_code, d_count_log)) != cudaSuccess ||
-        (e = launch_dep(true, k_cert_tail, 1, 1, 0, s, rc.sv_count, rc.sv_cap, dstats, d_ovf, d_counters, queue)) !=
+        (e = launch_dep(true, k_cert_tail, 1, 1, 0, s, rc.sv_count, rc.sv_cap, dstats, d_ovf, d_counters, queue, end)) !=
             cudaSuccess)
       return cuda_error(e, "detect fixed");
     ctx->launches += 6;

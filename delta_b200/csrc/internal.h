@@ -69,7 +69,36 @@ delta_status detect_run(delta_ctx *ctx, int driver, int precision, const delta_m
 // can take (detect.cu).
 cudaError_t detect_launch_limits(int driver, int *cull_per_sm, int *surv_per_sm);
 
-// Fixed-capacity (graph-capturable) detection (detect.cu).  `pose`: as for detect_run
+// End of a graph step, by one thread of the step's last kernel.  A step that integrated (no
+// overflow before it) is counted and logged; its counters (pend: candidate pairs, triangle
+// pairs, solved pairs, summed during the step) go to the running totals only if no overflow
+// arose in it either: the host repeats an overflowing step's detection, with its counters,
+// outside the graph, and the replays queued after it are frozen.  pend is cleared for the
+// next step.  step == null: not in a graph step.
+struct StepEnd {
+  const int *ovf_snap = nullptr, *ovf = nullptr;
+  const int64_t *n_contacts = nullptr;
+  int64_t *log = nullptr, log_len = 0;
+  int64_t *step = nullptr, *pend = nullptr, *pairs_total = nullptr, *counters = nullptr;
+#ifdef __CUDACC__
+  __device__ __forceinline__ void run() const {
+    if (!*ovf_snap) {
+      const int64_t k = *step;
+      if (k < log_len) log[k] = *n_contacts;
+      *step = k + 1;
+      if (!*(const volatile int *)ovf) {
+        *pairs_total += pend[0];
+        counters[0] += pend[1];
+        counters[1] += pend[2];
+      }
+    }
+    pend[0] = pend[1] = pend[2] = 0;
+  }
+#endif
+};
+
+// Fixed-capacity (graph-capturable) detection (detect.cu).  The culled drivers' last kernel
+// also ends the graph step when `end` is set.  `pose`: as for detect_run
 // (null: the certified driver reads the meshes' vertices and culls without body boxes).
 // `tri_bits`: bits of a triangle index within a body (every body has
 // fewer than 2^tri_bits triangles), used to pack the contact sort keys.
@@ -80,7 +109,8 @@ delta_status detect_fixed_init(cudaStream_t s, void *state, int64_t pair_cap, in
 delta_status detect_run_fixed(delta_ctx *ctx, cudaStream_t s, int driver, const delta_meshes &m, const int32_t *pa,
                               const int32_t *pb, int64_t pair_cap, const delta_contacts &out, int64_t *d_ncontacts,
                               int *d_ovf, int ovf_code, int64_t *d_counters, int64_t *d_count_log, void *state,
-                              void *temp, size_t temp_bytes, const Pose *pose = nullptr, int tri_bits = 16);
+                              void *temp, size_t temp_bytes, const Pose *pose = nullptr, int tri_bits = 16,
+                              const StepEnd &end = StepEnd{});
 
 // Thread-local last-error text (capi.cu).
 delta_status set_error(delta_status st, const std::string &msg);

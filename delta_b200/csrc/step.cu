@@ -5,6 +5,7 @@
 // contraction.  Summations that the reference performs sequentially (contacts of one
 // partner, then partners of one body) are kept sequential per pair / per body; no
 // floating-point atomics are used, so results do not depend on scheduling.
+#include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -165,25 +166,11 @@ __device__ __forceinline__ void contact_terms(const ContactView &cv, int64_t c, 
   Tc[2] = arm[0] * (f[1]) - arm[1] * (f[0]);
 }
 
-// Last kernel of a graph step.  A step that integrated (no overflow before it) is counted
-// and logged; its counters (pend: candidate pairs, triangle pairs, solved pairs, summed
-// during the step) go to the running totals only if no overflow arose in it either: the
-// host repeats an overflowing step's detection, with its counters, outside the graph, and
-// the replays queued after it are frozen.  pend is cleared for the next step.
-__global__ void k_step_end(const int *ovf_snap, const int *ovf, const int64_t *n_contacts, int64_t *log,
-                           int64_t log_len, int64_t *step, int64_t *pend, int64_t *pairs_total, int64_t *counters) {
+// Last kernel of a graph step of the plain driver (the culled drivers' last kernel ends
+// their steps).
+__global__ void k_step_end(StepEnd end) {
   dep_sync();
-  if (!*ovf_snap) {
-    const int64_t k = *step;
-    if (k < log_len) log[k] = *n_contacts;
-    *step = k + 1;
-    if (!*ovf) {
-      *pairs_total += pend[0];
-      counters[0] += pend[1];
-      counters[1] += pend[2];
-    }
-  }
-  pend[0] = pend[1] = pend[2] = 0;
+  end.run();
 }
 
 __global__ void k_segment_heads(ContactView cv, int64_t n, uint8_t *head) {
@@ -195,57 +182,94 @@ __global__ void k_segment_heads(ContactView cv, int64_t n, uint8_t *head) {
 // Partner-pair force sums, one thread per contact.  Every thread forms its contact's terms
 // for both sides (master: force and torque on the master; slave: with the inverted normal,
 // on the slave) in shared memory.  The thread at the first contact of a (master, slave)
-// segment then adds the segment's terms in contact order, forming itself the terms of
-// contacts past its block.  From 0.0 in contact order, these are the sums of the
-// getContactsForces loop over the pair's contacts (forces.cpp:23-396), bit for bit.
+// segment then adds the segment's terms in contact order.  From 0.0 in contact order, these
+// are the sums of the getContactsForces loop over the pair's contacts (forces.cpp:23-396),
+// bit for bit.  A block looks ahead 128 contacts: it finds the ends of its segments from
+// the heads' bit masks, and its threads form together the terms of the contacts past it
+// that belong to its last segment (the head used to walk the contacts to the end of its
+// segment, one load after another, and to form the terms past its block alone: 15 us of a
+// hopper step).
 //  - kFixed (graph path, count on the device): the sums go to entry 2c (on the master) and
-//    2c+1 (on the slave), c the segment's first contact, and the segment is counted in its
-//    slave's list.  Sums on obstacles are not formed: nothing reads them.
+//    2c+1 (on the slave), c the segment's first contact; the segment is counted in its
+//    slave's list; seg_next[c] is the first contact after it, plus kSameMaster when that
+//    has the same master, and master_run[i] = c + 1 for a master's first segment.  Sums on
+//    obstacles are not formed: nothing reads them.
 //  - otherwise: segment g (seg_start[g] == c) gets entries 2g and 2g+1, keyed
 //    (body << sh | partner) for the entry sort, sh the bits of a body index.
-constexpr int kHeadThreads = 128;
+constexpr int kHeadThreads = 128, kHeadSpan = 2 * kHeadThreads;
+constexpr uint32_t kSameMaster = 1u << 31;
 template <bool kFixed>
 __global__ void __launch_bounds__(kHeadThreads) k_pair_forces_heads(
     delta_scene s, ContactView cv, const int64_t *n_contacts_d, int64_t n_contacts_h, const int64_t *seg_start,
     const int64_t *n_seg_p, delta_step_params p, int sh, uint64_t *key, int64_t *val_idx, double *entry,
-    uint32_t *slave_count) {
+    uint32_t *slave_count, uint32_t *seg_next, uint32_t *master_run) {
   dep_sync();
-  __shared__ double term[12][kHeadThreads];  // master F, master T, slave F, slave T
+  __shared__ double term[12][kHeadSpan];  // master F, master T, slave F, slave T
+  __shared__ uint32_t heads[kHeadSpan / 32];
+  const int t = threadIdx.x;
   const int64_t blk0 = (int64_t)blockIdx.x * kHeadThreads;
-  const int64_t c = blk0 + threadIdx.x;
+  const int64_t c = blk0 + t;
   int64_t n = n_contacts_d ? *n_contacts_d : n_contacts_h;
   if (n > cv.cap) n = cv.cap;
   if (blk0 >= n) return;  // the whole block is past the contacts
-  const int64_t blk1 = blk0 + kHeadThreads < n ? blk0 + kHeadThreads : n;
-  int32_t i = 0, j = 0;
-  bool oi = true, oj = true;
-  if (c < n) {
-    i = cv.master[c];
-    j = cv.slave[c];
-    oi = kFixed && s.obstacle[i] != 0;
-    oj = kFixed && s.obstacle[j] != 0;
+  // heads of the block's contacts and of the next 128 (past the contacts: heads too)
+  int32_t ids[2][2];  // master, slave of contacts c and c + 128
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int64_t u = c + h * kHeadThreads;
+    bool head = true;
+    ids[h][0] = ids[h][1] = 0;
+    if (u < n) {
+      ids[h][0] = cv.master[u];
+      ids[h][1] = cv.slave[u];
+      head = u == 0 || ids[h][0] != cv.master[u - 1] || ids[h][1] != cv.slave[u - 1];
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, head);
+    if ((t & 31) == 0) heads[(t >> 5) + h * (kHeadThreads / 32)] = m;
+  }
+  __syncthreads();
+  // the first head after local contact x, kHeadSpan if there is none
+  auto next_head = [&](int x) {
+    for (int w = (x + 1) >> 5; w < kHeadSpan / 32; ++w) {
+      const uint32_t m = w == (x + 1) >> 5 ? heads[w] & (~0u << ((x + 1) & 31)) : heads[w];
+      if (m) return 32 * w + __ffs(m) - 1;
+    }
+    return kHeadSpan;
+  };
+  const int reach = next_head(kHeadThreads - 1);  // the block's last segment ends before this
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    const int64_t u = c + h * kHeadThreads;
+    if (u >= n || t + h * kHeadThreads >= (h ? reach : kHeadThreads)) continue;
+    const int32_t i = ids[h][0], j = ids[h][1];
+    const bool oi = kFixed && s.obstacle[i] != 0, oj = kFixed && s.obstacle[j] != 0;
     const BodyKin Ki = body_kin(s, i), Kj = body_kin(s, j);
     X Fc[3], Tc[3];
     if (!oi) {
-      contact_terms(cv, c, Ki, Kj, false, p, Fc, Tc);
+      contact_terms(cv, u, Ki, Kj, false, p, Fc, Tc);
       for (int k = 0; k < 3; ++k) {
-        term[k][threadIdx.x] = Fc[k].v;
-        term[3 + k][threadIdx.x] = Tc[k].v;
+        term[k][t + h * kHeadThreads] = Fc[k].v;
+        term[3 + k][t + h * kHeadThreads] = Tc[k].v;
       }
     }
     if (!oj) {
-      contact_terms(cv, c, Kj, Ki, true, p, Fc, Tc);
+      contact_terms(cv, u, Kj, Ki, true, p, Fc, Tc);
       for (int k = 0; k < 3; ++k) {
-        term[6 + k][threadIdx.x] = Fc[k].v;
-        term[9 + k][threadIdx.x] = Tc[k].v;
+        term[6 + k][t + h * kHeadThreads] = Fc[k].v;
+        term[9 + k][t + h * kHeadThreads] = Tc[k].v;
       }
     }
   }
   __syncthreads();
-  if (c >= n) return;
-  if (c > 0 && cv.master[c] == cv.master[c - 1] && cv.slave[c] == cv.slave[c - 1]) return;
-  int64_t c1 = c + 1;
-  while (c1 < n && cv.master[c1] == i && cv.slave[c1] == j) ++c1;
+  if (c >= n || !((heads[t >> 5] >> (t & 31)) & 1u)) return;
+  const int32_t i = ids[0][0], j = ids[0][1];
+  const bool oi = kFixed && s.obstacle[i] != 0, oj = kFixed && s.obstacle[j] != 0;
+  const int local = next_head(t);
+  int64_t c1 = blk0 + local;
+  if (local == kHeadSpan)  // a segment of more than 128 contacts
+    while (c1 < n && cv.master[c1] == i && cv.slave[c1] == j) ++c1;
+  if (c1 > n) c1 = n;
+  const int64_t span = blk0 + kHeadSpan;
   int64_t e0 = 2 * c;
   if constexpr (!kFixed) {
     int64_t lo = 0, hi = *n_seg_p;  // the segment index: seg_start[g] == c
@@ -255,20 +279,23 @@ __global__ void __launch_bounds__(kHeadThreads) k_pair_forces_heads(
       else hi = mid;
     }
     e0 = 2 * lo;
+  } else {
+    seg_next[c] = (uint32_t)c1 | (c1 < n && cv.master[c1] == i ? kSameMaster : 0u);
+    if (c == 0 || cv.master[c - 1] != i) master_run[i] = (uint32_t)c + 1u;
   }
-  // the sums of one side: terms from shared memory within the block, formed here past it
+  // the sums of one side: terms from shared memory, formed here past the look-ahead
   auto side = [&](int o, int32_t a, int32_t b, bool negate, int64_t e) {
     X F[3] = {X(0.0), X(0.0), X(0.0)}, T[3] = {X(0.0), X(0.0), X(0.0)};
-    for (int64_t u = c; u < c1 && u < blk1; ++u) {
-      const int t = (int)(u - blk0);
+    for (int64_t u = c; u < c1 && u < span; ++u) {
+      const int q = (int)(u - blk0);
       for (int k = 0; k < 3; ++k) {
-        F[k] += X(term[o + k][t]);
-        T[k] += X(term[o + 3 + k][t]);
+        F[k] += X(term[o + k][q]);
+        T[k] += X(term[o + 3 + k][q]);
       }
     }
-    if (c1 > blk1) {
+    if (c1 > span) {
       const BodyKin A = body_kin(s, a), B = body_kin(s, b);
-      for (int64_t u = blk1; u < c1; ++u) {
+      for (int64_t u = span; u < c1; ++u) {
         X Fc[3], Tc[3];
         contact_terms(cv, u, A, B, negate, p, Fc, Tc);
         for (int k = 0; k < 3; ++k) {
@@ -312,19 +339,23 @@ __global__ void k_fill_slave_lists(delta_scene s, ContactView cv, const int64_t 
 // (min, max), so a body's partners below it are the masters of the segments in which it is
 // the slave, and those above it the slaves of the segments in which it is the master.
 // The first come from the body's list, sorted by segment position (which orders them by
-// master); the second are the body's run of contacts as master, in contact order.  From
-// 0.0, these are the additions of the sorted-entry sums (k_body_forces), in that order.
-__global__ void k_body_forces_lists(delta_scene s, ContactView cv, const int64_t *n_contacts_d, const uint32_t *start,
-                                    int32_t *list, const double *entry, double *force, double *torque, uint8_t *has,
-                                    uint32_t *slave_count, uint32_t *fill) {
+// master); the second are the body's segments as master, in contact order, each naming the
+// next (walking the contacts of the run took a dependent load a contact, 13 to 18 us of a
+// hopper or box step).  From 0.0, these are the additions of the sorted-entry sums
+// (k_body_forces), in that order.
+__global__ void k_body_forces_lists(delta_scene s, const uint32_t *start, int32_t *list, const double *entry,
+                                    double *force, double *torque, uint8_t *has, uint32_t *slave_count,
+                                    uint32_t *fill, const uint32_t *seg_next, uint32_t *master_run) {
   dep_sync();
   const int32_t b = blockIdx.x * blockDim.x + threadIdx.x;
   const int32_t nb = s.n_bodies;
   if (b >= nb) return;
-  // the body's slave count and fill position, read by the kernels before this one, are
-  // cleared for the next step (slave_count[nb] is never counted)
+  const uint32_t run = master_run[b];  // 1 + the body's first contact as master, 0: none
+  // the body's slave count, fill position and run are cleared for the next step (their last
+  // reader; slave_count[nb] is never counted)
   slave_count[b] = 0u;
   fill[b] = 0u;
+  if (run) master_run[b] = 0u;
   X F[3] = {X(0.0), X(0.0), X(0.0)}, T[3] = {X(0.0), X(0.0), X(0.0)};
   bool any = false;
   auto add = [&](const double *v) {
@@ -345,16 +376,13 @@ __global__ void k_body_forces_lists(delta_scene s, ContactView cv, const int64_t
       }
       list[w] = v;
     }
+#pragma unroll 4
     for (uint32_t u = l0; u < l1; ++u) add(entry + (2 * (int64_t)list[u] + 1) * 6);
-    const int64_t n = *n_contacts_d < cv.cap ? *n_contacts_d : cv.cap;
-    int64_t lo = 0, hi = n;  // first contact with master >= b (masters ascend)
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (cv.master[mid] < b) lo = mid + 1;
-      else hi = mid;
+    for (uint32_t c = run; c != 0u;) {
+      const uint32_t next = seg_next[c - 1];
+      add(entry + 2 * (int64_t)(c - 1) * 6);
+      c = next & kSameMaster ? (next & ~kSameMaster) + 1u : 0u;
     }
-    for (int64_t c = lo; c < n && cv.master[c] == b; ++c)
-      if (c == lo || cv.slave[c] != cv.slave[c - 1]) add(entry + (2 * c) * 6);
   }
   for (int k = 0; k < 3; ++k) {
     force[(int64_t)k * nb + b] = F[k].v;
@@ -736,15 +764,13 @@ __device__ __forceinline__ void push_pair(int32_t a, int32_t b, int sh, uint64_t
 // pairs pushed, as (min, max) keys, are those of a search of all 27 cells for j > i.
 constexpr int kGridColumns = 5;
 
-__global__ void k_grid_pairs(delta_scene s, Grid g, HashGrid hg, int sh, uint64_t *out, unsigned long long *count,
-                             int64_t cap, double skin) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= kGridColumns * (int64_t)s.n_bodies) return;
-  const int32_t i = (int32_t)(t / kGridColumns), col = (int32_t)(t % kGridColumns);
+__device__ __forceinline__ void grid_column_pairs(const delta_scene &s, const HashGrid &hg, int32_t i, int32_t col,
+                                                  int sh, uint64_t *out, unsigned long long *count, int64_t cap,
+                                                  double skin) {
   if (s.obstacle[i]) return;
   // the body's cell from the key the count pass stored (coordinates modulo 2^kCellBits,
   // which is all cell_key keeps), instead of three FP64 divisions per thread
-  const uint64_t own = hg.cell[i];
+  const uint64_t own = __ldcg(hg.cell + i);
   const int64_t c[3] = {(int64_t)((own >> (2 * kCellBits)) & kCellMask), (int64_t)((own >> kCellBits) & kCellMask),
                         (int64_t)(own & kCellMask)};
   const int dx = col < 3 ? 1 : 0, dy = col < 3 ? col - 1 : (col == 3 ? 1 : 0);
@@ -754,12 +780,19 @@ __global__ void k_grid_pairs(delta_scene s, Grid g, HashGrid hg, int sh, uint64_
     const bool same = col == 4 && dz == 0;  // the body's own cell: only j > i
     const uint64_t key = cell_key(cx, cy, c[2] + dz);
     const uint32_t b = cell_bucket(key, hg.nb);
-    for (uint32_t q = hg.start[b]; q < hg.start[b + 1]; ++q) {
-      const int32_t j = hg.bodies[q];
-      if ((same ? j > i : j != i) && hg.cell[j] == key && spheres_within(s, i, j, skin))
+    for (uint32_t q = __ldcg(hg.start + b), e = __ldcg(hg.start + b + 1); q < e; ++q) {
+      const int32_t j = __ldcg(hg.bodies + q);
+      if ((same ? j > i : j != i) && __ldcg(hg.cell + j) == key && spheres_within(s, i, j, skin))
         push_pair(i, j, sh, out, count, cap);
     }
   }
+}
+
+__global__ void k_grid_pairs(delta_scene s, Grid g, HashGrid hg, int sh, uint64_t *out, unsigned long long *count,
+                             int64_t cap, double skin) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= kGridColumns * (int64_t)s.n_bodies) return;
+  grid_column_pairs(s, hg, (int32_t)(t / kGridColumns), (int32_t)(t % kGridColumns), sh, out, count, cap, skin);
 }
 
 // obstacle L (box lo/hi) against every moving body j
@@ -1050,7 +1083,7 @@ delta_status forces_run(delta_ctx *ctx, const delta_scene &s, const delta_contac
   if ((e = cudaMemsetAsync(key, 0xff, sizeof(uint64_t) * 2 * nc, st)) != cudaSuccess) return cuda_error(e, "memset");
   const int sh = bits_for(n);
   k_pair_forces_heads<false><<<blocks_for(n_contacts, kHeadThreads), kHeadThreads, 0, st>>>(
-      s, cv, nullptr, n_contacts, seg_start, n_seg, p, sh, key, idx, entry, nullptr);
+      s, cv, nullptr, n_contacts, seg_start, n_seg, p, sh, key, idx, entry, nullptr, nullptr, nullptr);
   ctx->launches += 1;
   tb = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tb, key, skey, idx, sidx, (int64_t)(2 * nc), 0, 2 * sh, st);
@@ -1275,7 +1308,7 @@ delta_status broadphase_run(delta_ctx *ctx, const delta_scene &s, const Broadpha
 
 // Forces from a fixed-capacity contact buffer with its count on the device.
 size_t forces_fixed_state_bytes(int64_t cap, int32_t n_bodies) {
-  return 4 * 256 + 96 * (size_t)cap + 4 * (size_t)cap + 4 * (2 * (size_t)n_bodies + 1) + 4 * ((size_t)n_bodies + 1);
+  return 5 * 256 + 96 * (size_t)cap + 8 * (size_t)cap + 4 * (3 * (size_t)n_bodies + 1) + 4 * ((size_t)n_bodies + 1);
 }
 
 size_t forces_fixed_temp_bytes(int64_t cap, int32_t n_bodies) {
@@ -1285,54 +1318,59 @@ size_t forces_fixed_temp_bytes(int64_t cap, int32_t n_bodies) {
   return b;
 }
 
-// The fixed-capacity force state: entries (2 per segment, 6 doubles), slave lists, slave
-// counts [n + 1] and fill positions [n] (adjacent), list starts [n + 1].
-static void forces_fixed_layout(void *state, int64_t cap, int32_t n, double *&entry, int32_t *&list, uint32_t *&cnt,
-                                uint32_t *&fill, uint32_t *&start) {
-  auto align = [](char *q) { return (char *)(((uintptr_t)q + 255) & ~(uintptr_t)255); };
-  char *b = align((char *)state);
-  entry = (double *)b;
-  b = align(b + 96 * (size_t)cap);
-  list = (int32_t *)b;
-  b = align(b + 4 * (size_t)cap);
-  cnt = (uint32_t *)b;
-  fill = cnt + n + 1;
-  b = align(b + 4 * (2 * (size_t)n + 1));
-  start = (uint32_t *)b;
-}
-
-// Once per allocation of the force state: slave counts and fill positions at zero.
-static cudaError_t forces_fixed_init(cudaStream_t st, void *state, int64_t cap, int32_t n) {
+// The fixed-capacity force state: entries (2 per segment, 6 doubles), slave lists, segment
+// links, then slave counts [n + 1], fill positions [n] and master runs [n] (adjacent: zero
+// between steps), list starts [n + 1].
+struct ForcesFixed {
   double *entry;
   int32_t *list;
-  uint32_t *cnt, *fill, *start;
-  forces_fixed_layout(state, cap, n, entry, list, cnt, fill, start);
-  return cudaMemsetAsync(cnt, 0, 4 * (2 * (size_t)n + 1), st);
+  uint32_t *seg_next, *cnt, *fill, *run, *start;
+};
+
+static ForcesFixed forces_fixed_layout(void *state, int64_t cap, int32_t n) {
+  auto align = [](char *q) { return (char *)(((uintptr_t)q + 255) & ~(uintptr_t)255); };
+  ForcesFixed f;
+  char *b = align((char *)state);
+  f.entry = (double *)b;
+  b = align(b + 96 * (size_t)cap);
+  f.list = (int32_t *)b;
+  f.seg_next = (uint32_t *)(f.list + cap);
+  b = align(b + 8 * (size_t)cap);
+  f.cnt = (uint32_t *)b;
+  f.fill = f.cnt + n + 1;
+  f.run = f.fill + n;
+  b = align(b + 4 * (3 * (size_t)n + 1));
+  f.start = (uint32_t *)b;
+  return f;
+}
+
+// Once per allocation of the force state: counts, fill positions and runs at zero.
+static cudaError_t forces_fixed_init(cudaStream_t st, void *state, int64_t cap, int32_t n) {
+  return cudaMemsetAsync(forces_fixed_layout(state, cap, n).cnt, 0, 4 * (3 * (size_t)n + 1), st);
 }
 
 delta_status forces_run_fixed(cudaStream_t st, const delta_scene &s, const delta_contacts &c, const int64_t *d_nc,
                               const delta_step_params &p, double *force, double *torque, uint8_t *has, void *state,
-                              void *temp, size_t temp_bytes, int &kernels) {
+                              void *temp, size_t temp_bytes, int &kernels, bool follows) {
   cudaError_t e;
   const int64_t cap = c.capacity;
   const int32_t n = s.n_bodies;
   ContactView cv{c.x, c.normal, c.depth, c.master, c.slave, c.friction, cap};
-  double *entry;
-  int32_t *list;
-  uint32_t *cnt, *fill, *start;
-  forces_fixed_layout(state, cap, n, entry, list, cnt, fill, start);
-  // cnt and fill are zero: cleared at allocation (forces_fixed_init) and by the per-body
-  // sums of the step before
-  k_pair_forces_heads<true><<<blocks_for(cap, kHeadThreads), kHeadThreads, 0, st>>>(
-      s, cv, d_nc, 0, nullptr, nullptr, p, 0, nullptr, nullptr, entry, cnt);
+  const ForcesFixed f = forces_fixed_layout(state, cap, n);
+  // cnt, fill and run are zero: cleared at allocation (forces_fixed_init) and by the
+  // per-body sums of the step before
+  // programmatic dependent launches (pdl.cuh), but for the first kernel of a graph
+  if ((e = launch_dep(follows, k_pair_forces_heads<true>, blocks_for(cap, kHeadThreads), kHeadThreads, 0, st, s, cv,
+                      d_nc, 0, nullptr, nullptr, p, 0, nullptr, nullptr, f.entry, f.cnt, f.seg_next, f.run)) !=
+      cudaSuccess)
+    return cuda_error(e, "forces fixed");
   size_t tb = temp_bytes;
-  // the kernels after the first start as programmatic dependent launches (pdl.cuh)
-  if ((e = exclusive_sum(temp, tb, cnt, start, (int64_t)n + 1, st, true)) != cudaSuccess)
+  if ((e = exclusive_sum(temp, tb, f.cnt, f.start, (int64_t)n + 1, st, true)) != cudaSuccess)
     return cuda_error(e, "slave list scan");
-  if ((e = launch_dep(true, k_fill_slave_lists, blocks_for(cap), 256, 0, st, s, cv, d_nc, start, fill, list)) !=
+  if ((e = launch_dep(true, k_fill_slave_lists, blocks_for(cap), 256, 0, st, s, cv, d_nc, f.start, f.fill, f.list)) !=
           cudaSuccess ||
-      (e = launch_dep(true, k_body_forces_lists, blocks_for(n), 256, 0, st, s, cv, d_nc, start, list, entry, force,
-                      torque, has, cnt, fill)) != cudaSuccess)
+      (e = launch_dep(true, k_body_forces_lists, blocks_for(n), 256, 0, st, s, f.start, f.list, f.entry, force,
+                      torque, has, f.cnt, f.fill, f.seg_next, f.run)) != cudaSuccess)
     return cuda_error(e, "forces fixed");
   kernels += 4;
   return cuda_error(cudaGetLastError(), "forces fixed");
@@ -1407,8 +1445,8 @@ struct SkinList {
   int64_t cap = 0;                          // entries of keys, raw, sel
   unsigned long long *raw_count = nullptr;  // pairs found by the last build (may exceed cap)
   int64_t *sel_count = nullptr;             // this step's pairs (multi-CTA filter)
-  int *need = nullptr;                      // nonzero: rebuild before this step's filter
-  unsigned long long *rebuilds = nullptr;   // builds run inside the graph
+  int *need = nullptr;                      // nonzero: rebuild before this step's filter (GraphState)
+  unsigned long long *rebuilds = nullptr;   // builds run inside the graph (GraphState)
   uint64_t *keys = nullptr;                 // [cap] sorted keys of the last build, ~0 after them
   uint64_t *raw = nullptr;                  // [cap] a build's keys as found
   uint64_t *sel = nullptr;                  // [cap] this step's keys (multi-CTA filter)
@@ -1423,8 +1461,6 @@ static SkinList carve_skin(void *mem, int32_t n, int64_t cap) {
   k.cap = cap;
   k.raw_count = (unsigned long long *)b;
   k.sel_count = (int64_t *)(b + 8);
-  k.rebuilds = (unsigned long long *)(b + 16);
-  k.need = (int *)(b + 24);
   k.keys = (uint64_t *)(b + 256);
   k.raw = k.keys + cap;
   k.sel = k.raw + cap;
@@ -1547,6 +1583,390 @@ __global__ void k_unpack_selected(const uint64_t *__restrict__ sel, const int64_
   } else {
     pa[t] = pb[t] = -1;
   }
+}
+
+// ---- the whole skin-list step in one cluster -------------------------------------------
+// One kernel, a cluster of 16 CTAs of 1024 threads (8 where 16 cannot be resident together;
+// the cluster's barrier is the hardware's), checks the bodies' displacements, rebuilds the
+// list if a body has moved too far, tests every entry and writes the step's pairs in order.
+// It replaces two kernels for the check, a conditional graph node (8 us a step whether or
+// not its body runs) and two kernels for the filter: 14 to 18 us a step, 4 to 6 now.
+//
+// The common step has one cluster barrier: every thread tests its entries while the check
+// is still open; each CTA sends its count and its check's outcome to the others (distributed
+// shared memory), and after the barrier all know whether the flags hold or the list has to
+// be rebuilt and tested again.
+//
+// A build keeps the bodies as records in bucket order (position and reach, cell key and
+// index), so that a search step is one load where the grid kernels follow three pointers;
+// every atomic's return value is the rank of its element, so that placing needs no second
+// one; and the pairs are ordered by a counting sort over their first body and a rank within
+// its run (a moving body's few neighbours; an obstacle's run may be long).
+constexpr int kSkinMaxCtas = 16, kSkinThreads = 1024;
+constexpr int kSkinRounds = 4;  // entries per thread
+constexpr int64_t kSkinClusterCap = (int64_t)8 * kSkinThreads * kSkinRounds;
+// Scenes of more bodies keep the conditional node: a build by 16 SMs takes too long there.
+constexpr int32_t kSkinClusterBodies = 1 << 16;
+constexpr int kSkinBoxes = 128;  // obstacle boxes staged at a time
+
+struct SkinRecord {
+  double x, y, z, reach;  // centre, radius + eps
+};
+struct SkinCell {
+  uint64_t key;
+  int64_t body;
+};
+
+// The cluster's build state, after the list in its buffer.  bcount and acount are zero
+// between builds.
+struct SkinBuild {
+  int64_t nb = 0;           // buckets
+  SkinRecord *rec;          // [n] moving bodies in bucket order
+  SkinCell *cell;           // [n]
+  uint32_t *brank;          // [n] a body's rank in its bucket
+  uint32_t *bcount, *bstart;  // [nb + 1]
+  uint32_t *acount, *astart;  // [n + 1] pairs by first body
+  uint32_t *arank;          // [cap] a raw key's rank in its run
+};
+
+static size_t skin_build_bytes(int32_t n, int64_t cap) {
+  return 64 + 52 * (size_t)n + 8 * ((size_t)grid_buckets(n) + 1) + 8 * ((size_t)n + 1) + 4 * (size_t)cap;
+}
+
+static SkinBuild carve_skin_build(void *mem, int32_t n, int64_t cap) {
+  SkinBuild b;
+  b.nb = grid_buckets(n);
+  char *p = (char *)(((uintptr_t)mem + 63) & ~(uintptr_t)63);
+  b.rec = (SkinRecord *)p;
+  b.cell = (SkinCell *)(b.rec + n);
+  b.bcount = (uint32_t *)(b.cell + n);  // bcount and acount adjacent: zeroed together
+  b.acount = b.bcount + b.nb + 1;
+  b.bstart = b.acount + n + 1;
+  b.astart = b.bstart + b.nb + 1;
+  b.brank = b.astart + n + 1;
+  b.arank = b.brank + n;
+  (void)cap;
+  return b;
+}
+
+struct SkinStepSmem {
+  int sum[kSkinMaxCtas];        // pairs found by each CTA
+  int need[kSkinMaxCtas];       // a body of its share moved too far
+  int warp[kSkinRounds * 32];   // this CTA's counts, exclusive sums after the scan
+  uint32_t part[kSkinMaxCtas];  // the build's scans: each CTA's total
+  uint32_t wsum[32];
+  double box[kSkinBoxes][7];    // obstacle boxes and eps
+};
+
+// The cluster's barrier (release and acquire: the CTAs' global writes before it are visible
+// after it; what another CTA wrote is read past L1).
+__device__ __forceinline__ void skin_sync() { cooperative_groups::this_cluster().sync(); }
+
+// start[i] = count[0] + ... + count[i-1] for i < n, by the cluster: a contiguous share per
+// CTA, a contiguous run per thread.
+__device__ __forceinline__ void cluster_exclusive_scan(SkinStepSmem &sm, const uint32_t *count, uint32_t *start,
+                                                       int64_t n) {
+  auto cl = cooperative_groups::this_cluster();
+  const int rank = (int)cl.block_rank(), ctas = (int)cl.num_blocks(), t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int64_t share = (n + ctas - 1) / ctas, run = (share + kSkinThreads - 1) / kSkinThreads;
+  const int64_t i0 = rank * share + t * run;
+  const int64_t end = (rank + 1) * share < n ? (rank + 1) * share : n, i1 = i0 + run < end ? i0 + run : end;
+  uint32_t own = 0;
+  for (int64_t i = i0; i < i1; ++i) own += __ldcg(count + i);
+  uint32_t incl = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) sm.wsum[w] = incl;
+  __syncthreads();
+  if (w == 0) {
+    uint32_t v = sm.wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += y;
+    }
+    sm.wsum[lane] = v;
+    const uint32_t total = __shfl_sync(0xffffffffu, v, 31);
+    if (lane < ctas) *cl.map_shared_rank(&sm.part[rank], lane) = total;
+  }
+  __syncthreads();
+  cl.sync();
+  uint32_t at = (w > 0 ? sm.wsum[w - 1] : 0u) + incl - own;
+  for (int c = 0; c < rank; ++c) at += sm.part[c];
+  for (int64_t i = i0; i < i1; ++i) {
+    start[i] = at;
+    at += __ldcg(count + i);
+  }
+  skin_sync();
+}
+
+// A pair of the build: its key and its rank among the pairs of its first body.
+__device__ __forceinline__ void push_ranked(int32_t a, int32_t b, int sh, const SkinList &k, const SkinBuild &bd) {
+  const int32_t lo = a < b ? a : b, hi = a < b ? b : a;
+  // one atomic on the shared counter per group of lanes that arrive together
+  const unsigned grp = __activemask();
+  const int lane = threadIdx.x & 31, leader = __ffs(grp) - 1;
+  unsigned long long pos = 0;
+  if (lane == leader) pos = atomicAdd(k.raw_count, (unsigned long long)__popc(grp));
+  const uint32_t rank = atomicAdd(&bd.acount[lo], 1u);
+  pos = __shfl_sync(grp, pos, leader) + __popc(grp & ((1u << lane) - 1u));
+  if ((int64_t)pos < k.cap) {
+    k.raw[pos] = ((uint64_t)(uint32_t)lo << sh) | (uint32_t)hi;
+    bd.arank[pos] = rank;
+  }
+}
+
+// The list rebuilt at the current positions: the pairs within reach + skin of skin_build's
+// search (k_grid_pairs, k_obstacle_pairs; the reaches are added in another order, which the
+// test's margins cover), in key order.
+__device__ __forceinline__ void cluster_skin_build(SkinStepSmem &sm, const delta_scene &s, const Grid &g,
+                                                   const SkinBuild &bd, const SkinList &k, int sh,
+                                                   const int32_t *obst, const double *box, int32_t n_obst,
+                                                   double skin, int *ovf) {
+  auto cl = cooperative_groups::this_cluster();
+  const int64_t t = (int64_t)cl.block_rank() * kSkinThreads + threadIdx.x, T = (int64_t)cl.num_blocks() * kSkinThreads;
+  const int32_t n = s.n_bodies;
+  // 1. cells, buckets and ranks
+  if (t == 0) *k.raw_count = 0ull;
+  for (int64_t i = t; i < n; i += T) {
+    if (s.obstacle[i]) continue;
+    int64_t c[3];
+    cell_of(s, g, (int32_t)i, c);
+    bd.brank[i] = atomicAdd(&bd.bcount[cell_bucket(cell_key(c[0], c[1], c[2]), bd.nb)], 1u);
+  }
+  skin_sync();
+  cluster_exclusive_scan(sm, bd.bcount, bd.bstart, bd.nb + 1);
+  // 2. records in bucket order (brank by the thread that wrote it)
+  for (int64_t i = t; i < n; i += T) {
+    if (s.obstacle[i]) continue;
+    int64_t c[3];
+    cell_of(s, g, (int32_t)i, c);
+    const uint64_t key = cell_key(c[0], c[1], c[2]);
+    const uint32_t at = __ldcg(bd.bstart + cell_bucket(key, bd.nb)) + bd.brank[i];
+    bd.rec[at] = SkinRecord{s.pos[i], s.pos[n + i], s.pos[2 * (int64_t)n + i], s.radius[i] + s.eps[i]};
+    bd.cell[at] = SkinCell{key, i};
+  }
+  skin_sync();
+  // 3. the search over half the neighbourhood (k_grid_pairs), five threads a body in bucket
+  // order; the obstacle boxes against every body
+  for (int64_t i = t; i < bd.nb + 1; i += T) bd.bcount[i] = 0u;
+  const int64_t moving = __ldcg(bd.bstart + bd.nb);
+  auto within = [&](double d2, double reach) {
+    reach = reach * (1.0 + 1e-9) + 1e-12;
+    reach = (reach + skin) * (1.0 + 1e-9) + 1e-12;
+    return d2 <= reach * reach;
+  };
+  auto load_rec = [&](int64_t q) {
+    const double2 *p = reinterpret_cast<const double2 *>(bd.rec + q);
+    const double2 u = __ldcg(p), v = __ldcg(p + 1);
+    return SkinRecord{u.x, u.y, v.x, v.y};
+  };
+  auto load_cell = [&](int64_t q) {
+    const longlong2 v = __ldcg(reinterpret_cast<const longlong2 *>(bd.cell + q));
+    return SkinCell{(uint64_t)v.x, v.y};
+  };
+  for (int64_t w = t; w < kGridColumns * moving; w += T) {
+    const int64_t e = w / kGridColumns;
+    const int col = (int)(w - e * kGridColumns);
+    const SkinCell own = load_cell(e);
+    const SkinRecord me = load_rec(e);
+    const int64_t c0 = (int64_t)((own.key >> (2 * kCellBits)) & kCellMask) + (col < 3 ? 1 : 0);
+    const int64_t c1 = (int64_t)((own.key >> kCellBits) & kCellMask) + (col < 3 ? col - 1 : (col == 3 ? 1 : 0));
+    const int64_t c2 = (int64_t)(own.key & kCellMask);
+    uint64_t key[3];
+    uint32_t q0[3], q1[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      key[d] = cell_key(c0, c1, c2 + d - 1);
+      const uint32_t b = cell_bucket(key[d], bd.nb);
+      const bool skip = col == 4 && d == 0;  // the own column: the own cell (bodies after this one) and dz = 1
+      q0[d] = skip ? 0u : __ldcg(bd.bstart + b);
+      q1[d] = skip ? 0u : __ldcg(bd.bstart + b + 1);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      for (uint32_t q = q0[d]; q < q1[d]; ++q) {
+        const SkinCell o = load_cell(q);
+        const SkinRecord r = load_rec(q);
+        if (o.key != key[d] || (col == 4 && d == 1 ? o.body <= own.body : o.body == own.body)) continue;
+        const double dx = r.x - me.x, dy = r.y - me.y, dz = r.z - me.z;
+        if (within(dx * dx + dy * dy + dz * dz, me.reach + r.reach))
+          push_ranked((int32_t)own.body, (int32_t)o.body, sh, k, bd);
+      }
+  }
+  for (int32_t o0 = 0; o0 < n_obst; o0 += kSkinBoxes) {
+    const int32_t no = n_obst - o0 < kSkinBoxes ? n_obst - o0 : kSkinBoxes;
+    __syncthreads();
+    for (int i = threadIdx.x; i < 7 * no; i += kSkinThreads)
+      sm.box[i / 7][i % 7] = i % 7 < 6 ? box[6 * (int64_t)(o0 + i / 7) + i % 7] : s.eps[obst[o0 + i / 7]];
+    __syncthreads();
+    for (int64_t e = t; e < moving; e += T) {
+      const SkinRecord me = load_rec(e);
+      const double c[3] = {me.x, me.y, me.z};
+      for (int32_t o = 0; o < no; ++o) {
+        double d2 = 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const double gap = fmax(sm.box[o][d] - c[d], c[d] - sm.box[o][3 + d]);
+          if (gap > 0.0) d2 += gap * gap;
+        }
+        if (within(d2, me.reach + sm.box[o][6])) push_ranked(obst[o0 + o], (int32_t)load_cell(e).body, sh, k, bd);
+      }
+    }
+  }
+  skin_sync();
+  // 4. the pairs in key order; a list that outgrew its capacity is left empty (the step is
+  // detected again by the host)
+  const int64_t found = (int64_t)__ldcg(k.raw_count), m = found <= k.cap ? found : 0;
+  if (t == 0 && found > k.cap) atomicCAS(ovf, 0, 1);
+  cluster_exclusive_scan(sm, bd.acount, bd.astart, (int64_t)n + 1);
+  for (int64_t i = t; i < n + 1; i += T) bd.acount[i] = 0u;
+  for (int64_t i = t; i < m; i += T) {
+    const uint64_t key = __ldcg(k.raw + i);
+    k.sel[__ldcg(bd.astart + (key >> sh)) + __ldcg(bd.arank + i)] = key;
+  }
+  skin_sync();
+  for (int64_t i = t; i < k.cap; i += T) {
+    if (i >= m) {
+      k.keys[i] = ~0ull;
+      continue;
+    }
+    const uint64_t key = __ldcg(k.sel + i);
+    const uint32_t lo = __ldcg(bd.astart + (key >> sh)), hi = __ldcg(bd.astart + (key >> sh) + 1);
+    uint32_t r = lo;
+#pragma unroll 8
+    for (uint32_t q = lo; q < hi; ++q) r += __ldcg(k.sel + q) < key ? 1u : 0u;
+    k.keys[r] = key;
+  }
+  for (int64_t i = t; i < 3 * (int64_t)n; i += T) k.anchor[i] = s.pos[i];
+  if (t == 0) {
+    *k.need = 0;
+    *k.rebuilds += 1ull;
+  }
+  skin_sync();
+}
+
+__global__ void __launch_bounds__(kSkinThreads, 1)
+    k_skin_step(delta_scene s, Grid g, SkinBuild bd, SkinList k, SkinTouch touch, const int32_t *obst, int32_t n_obst,
+                double skin, double limit2, int32_t *pa, int32_t *pb, int64_t pair_cap,
+                unsigned long long *count_out, int *ovf, int64_t *total) {
+  dep_sync();
+  __shared__ SkinStepSmem sm;
+  auto cl = cooperative_groups::this_cluster();
+  const int rank = (int)cl.block_rank(), ctas = (int)cl.num_blocks(), t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int32_t n = s.n_bodies;
+  // (the other CTAs must have started before their shared memory is written)
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  int moved = *(volatile const int *)k.need;  // set at the start of a call
+  for (int64_t i = (int64_t)rank * kSkinThreads + t; i < n; i += (int64_t)ctas * kSkinThreads) {
+    if (s.obstacle[i]) continue;
+    double d2 = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double d = s.pos[c * (int64_t)n + i] - k.anchor[c * (int64_t)n + i];
+      d2 += d * d;
+    }
+    if (!(d2 <= limit2)) moved = 1;
+  }
+  // this CTA's share of the list, round by round; a thread's flags and keys stay with it
+  const int64_t share = (k.cap + ctas - 1) / ctas;
+  const int rounds = (int)((share + kSkinThreads - 1) / kSkinThreads);
+  const int64_t base = rank * share, end = base + share < k.cap ? base + share : k.cap;
+  unsigned bal[kSkinRounds];
+  uint64_t key[kSkinRounds];
+  bool rebuilt = false;
+  for (;;) {
+#pragma unroll
+    for (int r = 0; r < kSkinRounds; ++r) {
+      bal[r] = 0u;
+      key[r] = ~0ull;
+      if (r < rounds) {
+        const int64_t i = base + (int64_t)r * kSkinThreads + t;
+        if (i < end) key[r] = __ldcg(k.keys + i);
+        // (a list that has yet to be built for the first time holds no keys)
+        bal[r] = __ballot_sync(0xffffffffu, touch(key[r]));
+        if (lane == 0) sm.warp[r * 32 + w] = __popc(bal[r]);
+      }
+    }
+    const int any = __syncthreads_or(!rebuilt && moved);
+    if (!rebuilt) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (w == 0) {
+      // exclusive sums of the rounds' warp counts, 32 at a time
+      int carry = 0;
+      for (int r = 0; r < rounds; ++r) {
+        const int v = sm.warp[r * 32 + lane];
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        sm.warp[r * 32 + lane] = carry + incl - v;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane < ctas) {
+        *cl.map_shared_rank(&sm.sum[rank], lane) = carry;
+        *cl.map_shared_rank(&sm.need[rank], lane) = any;
+      }
+    }
+    cl.sync();
+    int need = 0;
+    for (int c = 0; c < ctas; ++c) need |= sm.need[c];
+    if (!need) break;
+    cluster_skin_build(sm, s, g, bd, k, touch.sh, obst, touch.box, n_obst, skin, ovf);
+    rebuilt = true;  // (the build ends with a barrier: sum and need are free to be sent again)
+  }
+  int before = 0, found = 0;
+  for (int c = 0; c < ctas; ++c) {
+    before += c < rank ? sm.sum[c] : 0;
+    found += sm.sum[c];
+  }
+  const uint64_t low = (1ull << touch.sh) - 1ull;
+#pragma unroll
+  for (int r = 0; r < kSkinRounds; ++r)
+    if (r < rounds && ((bal[r] >> lane) & 1u)) {
+      const int pos = before + sm.warp[r * 32 + w] + __popc(bal[r] & ((1u << lane) - 1u));
+      if (pos < pair_cap) {
+        pa[pos] = (int32_t)(key[r] >> touch.sh);
+        pb[pos] = (int32_t)(key[r] & low);
+      }
+    }
+  for (int64_t i = found + (int64_t)rank * kSkinThreads + t; i < pair_cap; i += (int64_t)ctas * kSkinThreads)
+    pa[i] = pb[i] = -1;
+  if (rank == 0 && t == 0) {
+    *count_out = (unsigned long long)found;
+    if (found > pair_cap) atomicCAS(ovf, 0, 1);
+    if (total) *total += found < pair_cap ? found : pair_cap;
+  }
+}
+
+// Whether a scene's skin list is handled by one cluster.
+static bool skin_cluster(int32_t n, int64_t cap) { return cap > 0 && cap <= kSkinClusterCap && n <= kSkinClusterBodies; }
+
+// CTAs of k_skin_step's cluster: 16 (beyond the portable 8, so asked for) where they can be
+// resident together.
+static cudaError_t skin_cluster_size(int *ctas) {
+  cudaError_t e = cudaFuncSetAttribute(k_skin_step, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kSkinMaxCtas);
+  cfg.blockDim = dim3(kSkinThreads);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kSkinMaxCtas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, k_skin_step, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    clusters = 0;
+  }
+  *ctas = clusters >= 1 ? kSkinMaxCtas : 8;
+  return cudaSuccess;
 }
 
 static SkinTouch skin_touch(const delta_scene &s, const BroadphasePlan &plan) {
@@ -1679,6 +2099,17 @@ static cudaError_t skin_filter(cudaStream_t st, const delta_scene &s, const Broa
 // simulation object
 // ---------------------------------------------------------------------------------------
 
+// Device state of the replayed step, set by one copy at the start of a call and read back
+// with the step log (which follows it at +256) by one at its end.
+struct GraphState {
+  int64_t n_contacts, step, cnt[2];
+  int ovf, snap;
+  int64_t body_pairs, pend[3];
+  int need, pad;                // skin list: rebuild before the next filter
+  unsigned long long rebuilds;  // skin list: builds so far (kept from call to call)
+};
+static_assert(sizeof(GraphState) <= 256, "the log follows at +256");
+
 struct delta_sim {
   delta_ctx *ctx = nullptr;
   delta_scene scene{};
@@ -1719,6 +2150,7 @@ struct delta_sim {
     int64_t *d_nc = nullptr, *d_step = nullptr, *d_cnt = nullptr, *d_log = nullptr;
     int *d_ovf = nullptr, *d_snap = nullptr;
     int64_t *d_bp = nullptr;  // candidate body pairs summed over the replayed steps
+    GraphState *state = nullptr;  // what d_nc .. d_pend point into
     int64_t *d_pend = nullptr;  // the step in flight's pairs, triangle pairs, solved pairs
     int64_t log_len = 0;
     // the skin list (its buffer sk), its rebuilds' kernels, and the stream its conditional
@@ -1726,18 +2158,24 @@ struct delta_sim {
     void *sk = nullptr;
     delta::SkinList skin{};
     int rebuild_kernels = 0;
+    int skin_ctas = 8;  // k_skin_step's cluster
     unsigned long long rebuilds_seen = 0;
     cudaStream_t stream2 = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev = nullptr;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
+    // the recorded step, and kGraphSteps of it in one graph (recorded when a call has as many)
+    cudaGraph_t graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t exec[2] = {nullptr, nullptr};
     delta_step_params params{};
     int kernels = 0;
     int64_t launch_epoch = 0;  // the context's launch shapes the graph was recorded with
-    bool captured = false;
   } g;
 };
+
+// Steps of the longer recorded graph.  Between two graph launches the GPU idles for about 4
+// us (a replayed lattice step is 46); inside a graph a step's first kernel starts as a
+// dependent launch like the others.
+static constexpr int kGraphSteps = 8;
 
 namespace delta {
 
@@ -1835,12 +2273,17 @@ static delta_status sim_detect(delta_sim *s) {
   return DELTA_OK;
 }
 
+static void graph_drop_recorded(delta_sim::Graph &g) {
+  for (int k = 0; k < 2; ++k) {
+    if (g.exec[k]) cudaGraphExecDestroy(g.exec[k]);
+    if (g.graph[k]) cudaGraphDestroy(g.graph[k]);
+    g.exec[k] = nullptr;
+    g.graph[k] = nullptr;
+  }
+}
+
 static void graph_release(delta_sim::Graph &g) {
-  if (g.exec) cudaGraphExecDestroy(g.exec);
-  if (g.graph) cudaGraphDestroy(g.graph);
-  g.exec = nullptr;
-  g.graph = nullptr;
-  g.captured = false;
+  graph_drop_recorded(g);
   for (void *p : {(void *)g.pa, g.bp, g.fs, g.ds, g.temp, g.c_mem, g.dev, g.sk})
     if (p) cudaFree(p);
   g.pa = g.pb = nullptr;
@@ -1877,15 +2320,15 @@ static delta_status graph_alloc(delta_sim *s, int64_t pair_cap, int64_t contact_
                        (int32_t *)(d + 14 * cap), (int32_t *)(d + 14 * cap) + cap,
                        (int32_t *)(d + 14 * cap) + 2 * cap, (int32_t *)(d + 14 * cap) + 3 * cap,
                        (int32_t *)(d + 14 * cap) + 4 * cap, (uint8_t *)((int32_t *)(d + 14 * cap) + 5 * cap)};
-  char *v = (char *)g.dev;
-  g.d_nc = (int64_t *)v;
-  g.d_step = (int64_t *)(v + 8);
-  g.d_cnt = (int64_t *)(v + 16);
-  g.d_ovf = (int *)(v + 32);
-  g.d_snap = (int *)(v + 36);
-  g.d_bp = (int64_t *)(v + 40);
-  g.d_pend = (int64_t *)(v + 48);  // 3 counters of the step in flight
-  g.d_log = (int64_t *)(v + 256);
+  g.state = (GraphState *)g.dev;
+  g.d_nc = &g.state->n_contacts;
+  g.d_step = &g.state->step;
+  g.d_cnt = g.state->cnt;
+  g.d_ovf = &g.state->ovf;
+  g.d_snap = &g.state->snap;
+  g.d_bp = &g.state->body_pairs;
+  g.d_pend = g.state->pend;  // 3 counters of the step in flight
+  g.d_log = (int64_t *)((char *)g.dev + 256);
   if ((e = cudaMemset(g.dev, 0, 256)) != cudaSuccess) return cuda_error(e, "graph memset");
   if ((e = block_sort_prepare()) != cudaSuccess) return cuda_error(e, "pair sort attributes");
   if ((e = forces_fixed_init(s->ctx->stream, g.fs, contact_cap, n)) != cudaSuccess) return cuda_error(e, "forces init");
@@ -1904,13 +2347,39 @@ static delta_status graph_alloc(delta_sim *s, int64_t pair_cap, int64_t contact_
       if ((e = cudaMalloc(&g.temp, tb)) != cudaSuccess) return cuda_error(e, "skin temp");
       g.temp_bytes = tb;
     }
-    if ((e = cudaMalloc(&g.sk, skin_bytes(n, cap))) != cudaSuccess) return cuda_error(e, "skin list");
+    const bool cluster = skin_cluster(n, cap);
+    if ((e = cudaMalloc(&g.sk, skin_bytes(n, cap) + (cluster ? skin_build_bytes(n, cap) : 0))) != cudaSuccess)
+      return cuda_error(e, "skin list");
     g.skin = carve_skin(g.sk, n, cap);
-    if ((e = cudaMemset(g.sk, 0, 256)) != cudaSuccess || (e = cudaMemset(g.skin.need, 0xff, sizeof(int))) != cudaSuccess)
+    if (cluster) {
+      const SkinBuild bd = carve_skin_build(g.skin.anchor + 3 * (size_t)n, n, cap);
+      if ((e = cudaMemset(bd.bcount, 0, 4 * ((size_t)bd.nb + n + 2))) != cudaSuccess ||
+          (e = skin_cluster_size(&g.skin_ctas)) != cudaSuccess)
+        return cuda_error(e, "skin build state");
+    }
+    g.skin.need = &g.state->need;
+    g.skin.rebuilds = &g.state->rebuilds;
+    // (keys: all empty until the first build, because k_skin_step tests them before it)
+    if ((e = cudaMemset(g.sk, 0, 256)) != cudaSuccess || (e = cudaMemset(g.skin.need, 0xff, sizeof(int))) != cudaSuccess ||
+        (e = cudaMemset(g.skin.keys, 0xff, sizeof(uint64_t) * (size_t)cap)) != cudaSuccess)
       return cuda_error(e, "skin init");
   }
   if ((e = cudaStreamSynchronize(s->ctx->stream)) != cudaSuccess) return cuda_error(e, "graph init");
   return DELTA_OK;
+}
+
+// The step's broadphase from the skin list by one cluster, under capture on g.stream.
+static delta_status graph_skin_cluster(delta_sim *s, int &k) {
+  delta_sim::Graph &g = s->g;
+  const BroadphasePlan &plan = s->plan;
+  const double limit = 0.5 * plan.skin * (1.0 - 1e-9);
+  const cudaError_t e = launch_dep_cluster(
+      k_skin_step, (unsigned)g.skin_ctas, kSkinThreads, g.stream, s->scene, plan.gs,
+      carve_skin_build(g.skin.anchor + 3 * (size_t)s->scene.n_bodies, s->scene.n_bodies, g.skin.cap), g.skin,
+      skin_touch(s->scene, plan), plan.d_obst, plan.n_obst, plan.skin, limit * limit, g.pa, g.pb, g.pair_cap,
+      broadphase_fixed_count(g.bp, s->scene.n_bodies), g.d_ovf, g.d_pend);
+  k += 1;
+  return cuda_error(e, "skin step");
 }
 
 // The step's broadphase from the skin list, under capture on g.stream: the check sets
@@ -1962,29 +2431,28 @@ static delta_status graph_skin_broadphase(delta_sim *s, int &k) {
 
 // The skin list's rebuilds inside the graph since the last count: their kernels go to the
 // context's launch count, the builds to the simulation's total.
-static delta_status graph_count_rebuilds(delta_sim *s) {
+static void graph_count_rebuilds(delta_sim *s, unsigned long long rb) {
   delta_sim::Graph &g = s->g;
-  if (g.skin.cap <= 0) return DELTA_OK;
-  unsigned long long rb = 0;
-  cudaError_t e = cudaMemcpy(&rb, g.skin.rebuilds, 8, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_error(e, "skin rebuilds");
+  if (g.skin.cap <= 0) return;
   s->ctx->launches += (int64_t)(rb - g.rebuilds_seen) * g.rebuild_kernels;
   s->skin_rebuilds += (int64_t)(rb - g.rebuilds_seen);
   g.rebuilds_seen = rb;
-  return DELTA_OK;
 }
 
-// Enqueues one fixed-capacity step on g.stream (used under capture).
-static delta_status graph_enqueue_step(delta_sim *s, const delta_step_params &p) {
+// Enqueues one fixed-capacity step on g.stream (used under capture); `follows`: after another.
+static delta_status graph_enqueue_step(delta_sim *s, const delta_step_params &p, bool follows) {
   delta_sim::Graph &g = s->g;
   cudaStream_t st = g.stream;
   int k = 0;
-  delta_status ds = forces_run_fixed(st, s->scene, g.c, g.d_nc, p, s->F, s->T, s->has, g.fs, g.temp, g.temp_bytes, k);
+  delta_status ds = forces_run_fixed(st, s->scene, g.c, g.d_nc, p, s->F, s->T, s->has, g.fs, g.temp, g.temp_bytes, k,
+                                     follows);
   if (ds != DELTA_OK) return ds;
   cudaError_t le = launch_dep(true, k_bodies, blocks_for(s->scene.n_bodies, 128), 128, 0, st, s->scene, p, s->F, s->T,
                               s->has, g.d_ovf, g.d_snap, s->epoch);
   if (le != cudaSuccess) return cuda_error(le, "body update");
-  if (g.skin.cap > 0) {
+  if (skin_cluster(s->scene.n_bodies, g.skin.cap)) {
+    if ((ds = graph_skin_cluster(s, k)) != DELTA_OK) return ds;
+  } else if (g.skin.cap > 0) {
     if ((ds = graph_skin_broadphase(s, k)) != DELTA_OK) return ds;
   } else if ((ds = broadphase_run_fixed(st, s->scene, s->plan, g.pa, g.pb, g.pair_cap, g.d_ovf, g.d_pend, g.bp,
                                         g.temp, g.temp_bytes, k)) != DELTA_OK) {
@@ -2006,27 +2474,29 @@ static delta_status graph_enqueue_step(delta_sim *s, const delta_step_params &p)
   delta_meshes m{s->scene.n_bodies, s->scene.tri_offset, s->scene.x, s->scene.y, s->scene.z,
                  s->scene.eps,      s->scene.friction,   s->ids};
   const int64_t before = s->ctx->launches;
+  const StepEnd end{g.d_snap, g.d_ovf, g.d_nc, g.d_log, g.log_len, g.d_step, g.d_pend, g.d_bp, g.d_cnt};
   if ((ds = detect_run_fixed(s->ctx, st, s->driver, m, g.pa, g.pb, g.pair_cap, g.c, g.d_nc, g.d_ovf, 1, g.d_pend + 1,
-                             nullptr, g.ds, g.temp, g.temp_bytes, posed ? &pose : nullptr, s->tri_bits)) != DELTA_OK)
+                             nullptr, g.ds, g.temp, g.temp_bytes, posed ? &pose : nullptr, s->tri_bits,
+                             posed ? end : StepEnd{})) != DELTA_OK)
     return ds;
   k += (int)(s->ctx->launches - before);
   s->ctx->launches = before;
-  const cudaError_t ee = launch_dep(true, k_step_end, 1, 1, 0, st, g.d_snap, g.d_ovf, g.d_nc, g.d_log, g.log_len,
-                                    g.d_step, g.d_pend, g.d_bp, g.d_cnt);
-  if (ee != cudaSuccess) return cuda_error(ee, "step end");
-  g.kernels = k + 2;
+  if (!posed) {
+    const cudaError_t ee = launch_dep(true, k_step_end, 1, 1, 0, st, end);
+    if (ee != cudaSuccess) return cuda_error(ee, "step end");
+    k += 1;
+  }
+  g.kernels = k + 1;
   return cuda_error(cudaGetLastError(), "graph step");
 }
 
-static delta_status graph_capture(delta_sim *s, const delta_step_params &p) {
+// Records the step (which = 0) or kGraphSteps steps (1).
+static delta_status graph_capture(delta_sim *s, const delta_step_params &p, int which) {
   delta_sim::Graph &g = s->g;
-  if (g.exec) cudaGraphExecDestroy(g.exec);
-  if (g.graph) cudaGraphDestroy(g.graph);
-  g.exec = nullptr;
-  g.graph = nullptr;
   cudaError_t e = cudaStreamBeginCapture(g.stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_error(e, "begin capture");
-  delta_status ds = graph_enqueue_step(s, p);
+  delta_status ds = DELTA_OK;
+  for (int k = 0; k < (which ? kGraphSteps : 1) && ds == DELTA_OK; ++k) ds = graph_enqueue_step(s, p, k > 0);
   cudaGraph_t graph = nullptr;
   e = cudaStreamEndCapture(g.stream, &graph);
   if (ds != DELTA_OK) {
@@ -2034,32 +2504,46 @@ static delta_status graph_capture(delta_sim *s, const delta_step_params &p) {
     return ds;
   }
   if (e != cudaSuccess) return cuda_error(e, "end capture");
-  g.graph = graph;
-  if ((e = cudaGraphInstantiate(&g.exec, g.graph, 0)) != cudaSuccess) return cuda_error(e, "graph instantiate");
+  g.graph[which] = graph;
+  if ((e = cudaGraphInstantiate(&g.exec[which], graph, 0)) != cudaSuccess) return cuda_error(e, "graph instantiate");
   g.params = p;
   g.launch_epoch = s->ctx->launch_epoch;
-  g.captured = true;
   return DELTA_OK;
 }
 
-// Host contact list (sim->c) <-> graph contact buffer.
-static delta_status copy_contacts(const delta_contacts &src, const delta_contacts &dst, int64_t n, cudaStream_t st) {
-  cudaError_t e = cudaSuccess;
+// The first n contacts (n on the host, or on the device) of src into dst, as far as dst
+// holds them: one launch (20 copies took the host 80 us at either end of a call).
+__global__ void k_copy_contacts(delta_contacts src, delta_contacts dst, int64_t n_h, const int64_t *n_d) {
+  int64_t n = n_d ? *n_d : n_h;
+  if (n > src.capacity) n = src.capacity;
+  if (n > dst.capacity) n = dst.capacity;
   const int64_t ic = src.capacity, oc = dst.capacity;
-  for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
-    e = cudaMemcpyAsync(dst.x + k * oc, src.x + k * ic, 8 * n, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dst.normal + k * oc, src.normal + k * ic, 8 * n, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dst.P + k * oc, src.P + k * ic, 8 * n, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dst.Q + k * oc, src.Q + k * ic, 8 * n, cudaMemcpyDeviceToDevice, st);
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      dst.x[k * oc + c] = src.x[k * ic + c];
+      dst.normal[k * oc + c] = src.normal[k * ic + c];
+      dst.P[k * oc + c] = src.P[k * ic + c];
+      dst.Q[k * oc + c] = src.Q[k * ic + c];
+    }
+    dst.depth[c] = src.depth[c];
+    dst.eps_total[c] = src.eps_total[c];
+    dst.master[c] = src.master[c];
+    dst.slave[c] = src.slave[c];
+    dst.tri_a[c] = src.tri_a[c];
+    dst.tri_b[c] = src.tri_b[c];
+    dst.penetration[c] = src.penetration[c];
+    dst.friction[c] = src.friction[c];
   }
-  const void *srcs[] = {src.depth, src.eps_total, src.master, src.slave, src.tri_a, src.tri_b, src.penetration,
-                        src.friction};
-  void *dsts[] = {dst.depth, dst.eps_total, dst.master, dst.slave, dst.tri_a, dst.tri_b, dst.penetration,
-                  dst.friction};
-  const size_t sz[] = {8, 8, 4, 4, 4, 4, 4, 1};
-  for (int k = 0; k < 8 && e == cudaSuccess; ++k)
-    e = cudaMemcpyAsync(dsts[k], srcs[k], sz[k] * n, cudaMemcpyDeviceToDevice, st);
-  return cuda_error(e, "copy contacts");
+}
+
+static delta_status copy_contacts(const delta_contacts &src, const delta_contacts &dst, int64_t n, const int64_t *n_d,
+                                  cudaStream_t st) {
+  const int64_t most = n_d ? src.capacity : n;
+  if (most <= 0) return DELTA_OK;
+  const unsigned blocks = (unsigned)std::min<int64_t>((most + 255) / 256, 8 * kNumSMs);
+  k_copy_contacts<<<blocks, 256, 0, st>>>(src, dst, n, n_d);
+  return cuda_error(cudaGetLastError(), "copy contacts");
 }
 
 }  // namespace delta
@@ -2377,45 +2861,64 @@ delta_status delta_sim_step_graph(delta_sim *s, const delta_step_params *params,
                           std::max<int64_t>({g.log_len, (int64_t)nsteps, 4096}))) != DELTA_OK)
       return ds;
   }
-  if (memcmp(&g.params, params, sizeof(*params)) != 0 || g.launch_epoch != s->ctx->launch_epoch) g.captured = false;
+  if (memcmp(&g.params, params, sizeof(*params)) != 0 || g.launch_epoch != s->ctx->launch_epoch) graph_drop_recorded(g);
   // hand the current contacts to the graph buffers; ctx stream work must be done first
   if ((e = cudaEventRecord(g.ev, s->ctx->stream)) != cudaSuccess ||
       (e = cudaStreamWaitEvent(g.stream, g.ev, 0)) != cudaSuccess)
     return cuda_error(e, "graph order");
-  if ((ds = copy_contacts(s->c, g.c, s->n_contacts, g.stream)) != DELTA_OK) return ds;
-  int64_t hv[2] = {s->n_contacts, 0};
-  if ((e = cudaMemcpyAsync(g.d_nc, &hv[0], 8, cudaMemcpyHostToDevice, g.stream)) != cudaSuccess ||
-      (e = cudaMemsetAsync(g.d_step, 0, 8, g.stream)) != cudaSuccess ||
-      (e = cudaMemsetAsync(g.d_cnt, 0, 16, g.stream)) != cudaSuccess ||
-      (e = cudaMemsetAsync(g.d_bp, 0, 8, g.stream)) != cudaSuccess ||
-      (e = cudaMemsetAsync(g.d_pend, 0, 24, g.stream)) != cudaSuccess ||
-      (e = cudaMemsetAsync(g.d_ovf, 0, 8, g.stream)) != cudaSuccess ||
-      (g.skin.cap > 0 && (e = cudaMemsetAsync(g.skin.need, 0xff, sizeof(int), g.stream)) != cudaSuccess) ||
-      (e = cudaStreamSynchronize(g.stream)) != cudaSuccess)
+  void *pin = nullptr;
+  const size_t back_bytes = 256 + sizeof(int64_t) * (size_t)nsteps;
+  if ((ds = ctx_pinned(s->ctx, back_bytes, &pin)) != DELTA_OK) return ds;
+  if ((ds = copy_contacts(s->c, g.c, s->n_contacts, nullptr, g.stream)) != DELTA_OK) return ds;
+  s->ctx->launches += 1;
+  GraphState *host = (GraphState *)pin;
+  *host = GraphState{};
+  host->n_contacts = s->n_contacts;
+  host->need = -1;
+  if ((e = cudaMemcpyAsync(g.state, host, offsetof(GraphState, rebuilds), cudaMemcpyHostToDevice, g.stream)) !=
+      cudaSuccess)
     return cuda_error(e, "graph setup");
   int32_t base = done;  // steps completed before the current batch of launches
   while (done < nsteps) {
-    if (!g.captured && (ds = graph_capture(s, *params)) != DELTA_OK) return ds;
     const int32_t batch = nsteps - done;
-    for (int32_t k = 0; k < batch; ++k)
-      if ((e = cudaGraphLaunch(g.exec, g.stream)) != cudaSuccess) return cuda_error(e, "graph launch");
+    for (int32_t k = 0; k < batch;) {
+      const int which = batch - k >= kGraphSteps ? 1 : 0;
+      if (!g.exec[which] && (ds = graph_capture(s, *params, which)) != DELTA_OK) return ds;
+      if ((e = cudaGraphLaunch(g.exec[which], g.stream)) != cudaSuccess) return cuda_error(e, "graph launch");
+      k += which ? kGraphSteps : 1;
+    }
     s->ctx->launches += (int64_t)g.kernels * batch;
-    int64_t dev_step = 0;
-    int ovf = 0;
-    if ((e = cudaMemcpyAsync(&dev_step, g.d_step, 8, cudaMemcpyDeviceToHost, g.stream)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&ovf, g.d_ovf, 4, cudaMemcpyDeviceToHost, g.stream)) != cudaSuccess ||
+    // contacts back to the simulation, vertices up to date, state and log to the host: with
+    // the steps in one go (a step that overflowed is detected again below)
+    if ((ds = copy_contacts(g.c, s->c, 0, g.d_nc, g.stream)) != DELTA_OK ||
+        (ds = sim_all_vertices(s, g.stream)) != DELTA_OK)
+      return ds;
+    s->ctx->launches += 1;
+    if ((ds = ctx_pinned(s->ctx, back_bytes, &pin)) != DELTA_OK) return ds;
+    host = (GraphState *)pin;
+    const int64_t *log = (const int64_t *)((const char *)pin + 256);
+    if ((e = cudaMemcpyAsync(pin, g.dev, 256 + sizeof(int64_t) * (size_t)batch, cudaMemcpyDeviceToHost, g.stream)) !=
+            cudaSuccess ||
         (e = cudaStreamSynchronize(g.stream)) != cudaSuccess)
       return cuda_error(e, "graph sync");
+    const int64_t dev_step = host->step;
+    const int ovf = host->ovf;
     // dev_step counts graph steps (since setup) whose integration ran
     if (contacts_per_step) {
       const int64_t first = done - base;
       const int64_t n = dev_step - first;
-      if (n > 0 && (e = cudaMemcpy(contacts_per_step + done, g.d_log + first, 8 * n, cudaMemcpyDeviceToHost)) != cudaSuccess)
-        return cuda_error(e, "graph log");
+      if (n > 0) memcpy(contacts_per_step + done, log + first, 8 * (size_t)n);
     }
     s->counters[0] += dev_step - (done - base);
     done = base + (int32_t)dev_step;
-    if (!ovf) break;
+    s->counters[1] += host->body_pairs;
+    s->counters[2] += host->cnt[0];
+    s->counters[3] += host->cnt[1];
+    graph_count_rebuilds(s, host->rebuilds);
+    if (!ovf) {
+      s->n_contacts = host->n_contacts;
+      break;
+    }
     // overflow in the detection of the last integrated step: grow, detect again, recapture
     unsigned long long pc = 0;
     if ((e = cudaMemcpy(&pc, broadphase_fixed_count(g.bp, s->scene.n_bodies), 8, cudaMemcpyDeviceToHost)) !=
@@ -2424,39 +2927,25 @@ delta_status delta_sim_step_graph(delta_sim *s, const delta_step_params *params,
     if ((e = cudaStreamSynchronize(s->ctx->stream)) != cudaSuccess) return cuda_error(e, "sync");
     if ((ds = sim_detect(s)) != DELTA_OK) return ds;  // non-graph detection of the current state
     if (contacts_per_step && done > 0) contacts_per_step[done - 1] = s->n_contacts;
-    int64_t saved_log = g.log_len, seg_cnt[2] = {0, 0}, seg_bp = 0;
-    if ((e = cudaMemcpy(seg_cnt, g.d_cnt, 16, cudaMemcpyDeviceToHost)) != cudaSuccess ||
-        (e = cudaMemcpy(&seg_bp, g.d_bp, 8, cudaMemcpyDeviceToHost)) != cudaSuccess)
-      return cuda_error(e, "counters");
-    s->counters[1] += seg_bp;
-    s->counters[2] += seg_cnt[0];
-    s->counters[3] += seg_cnt[1];
-    if ((ds = graph_count_rebuilds(s)) != DELTA_OK) return ds;
+    const int64_t saved_log = g.log_len;
     if ((ds = graph_alloc(s, std::max<int64_t>(2 * g.pair_cap, 2 * (int64_t)pc), std::max<int64_t>(2 * g.contact_cap,
                           4 * s->n_contacts), saved_log)) != DELTA_OK)
       return ds;
-    if ((ds = copy_contacts(s->c, g.c, s->n_contacts, g.stream)) != DELTA_OK) return ds;
-    hv[0] = s->n_contacts;
-    if ((e = cudaMemcpyAsync(g.d_nc, &hv[0], 8, cudaMemcpyHostToDevice, g.stream)) != cudaSuccess ||
+    if ((ds = copy_contacts(s->c, g.c, s->n_contacts, nullptr, g.stream)) != DELTA_OK) return ds;
+    s->ctx->launches += 1;
+    if ((e = cudaMemcpyAsync(g.d_nc, &s->n_contacts, 8, cudaMemcpyHostToDevice, g.stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(g.stream)) != cudaSuccess)
       return cuda_error(e, "graph restart");
     base = done;
+    if (done >= nsteps && (ds = sim_all_vertices(s, g.stream)) != DELTA_OK) return ds;
   }
-  // counters and contacts back to the simulation object
-  int64_t cnt[2] = {0, 0}, nc = 0, bp = 0;
-  if ((e = cudaMemcpy(cnt, g.d_cnt, 16, cudaMemcpyDeviceToHost)) != cudaSuccess ||
-      (e = cudaMemcpy(&bp, g.d_bp, 8, cudaMemcpyDeviceToHost)) != cudaSuccess ||
-      (e = cudaMemcpy(&nc, g.d_nc, 8, cudaMemcpyDeviceToHost)) != cudaSuccess)
-    return cuda_error(e, "graph counters");
-  s->counters[1] += bp;
-  s->counters[2] += cnt[0];
-  s->counters[3] += cnt[1];
-  if ((ds = graph_count_rebuilds(s)) != DELTA_OK) return ds;
-  if (nc > s->c.capacity && (ds = alloc_contacts(s, nc + nc / 2 + 1024)) != DELTA_OK) return ds;
-  if ((ds = copy_contacts(g.c, s->c, nc, g.stream)) != DELTA_OK) return ds;
-  if ((ds = sim_all_vertices(s, g.stream)) != DELTA_OK) return ds;
+  if (s->n_contacts > s->c.capacity) {  // more than the simulation's buffer held
+    const int64_t nc = s->n_contacts;
+    if ((ds = alloc_contacts(s, nc + nc / 2 + 1024)) != DELTA_OK) return ds;
+    if ((ds = copy_contacts(g.c, s->c, nc, nullptr, g.stream)) != DELTA_OK) return ds;
+    s->ctx->launches += 1;
+  }
   if ((e = cudaStreamSynchronize(g.stream)) != cudaSuccess) return cuda_error(e, "graph end");
-  s->n_contacts = nc;
   return DELTA_OK;
 }
 

@@ -514,3 +514,55 @@ def test_graph_skin_list_overflow_recovers(ctx):
     assert skin["capacity"] > 1024 + 1024 // 2, skin  # grown past the first list
     assert sum(stepped[0]) > 0
     _assert_same_run(stepped, graph)
+
+
+@pytest.mark.parametrize("kind", ["few", "many_obstacles", "dense"])
+def test_graph_skin_cluster_equals_stepping(ctx, kind):
+    """The skin list's cluster kernel against delta_sim_step, bit for bit with counters, over
+    rebuilds: 3 bodies (most threads idle); 256 obstacle boxes (staged 128 at a time); a
+    close-packed cloud whose list takes the cluster more than one round (above 16,384)."""
+    from delta_b200.engine import StepParams
+    from delta_b200.scenarios import hopper_obstacles, particle_cloud_scene
+
+    rng = np.random.default_rng(23)
+    if kind == "few":
+        cen, obst = np.array([[0.0, 0.02, 0.0], [0.021, 0.02, 0.0], [0.0, 0.041, 0.0]]), []
+    elif kind == "many_obstacles":
+        th, y = rng.uniform(0, 2 * np.pi, 600), rng.uniform(0.1, 0.7, 600)
+        r = 0.03 + y * np.tan(np.radians(30.0))
+        cen, obst = np.stack([r * np.cos(th), y, r * np.sin(th)], 1), hopper_obstacles(patch=(2, 2))
+        assert len(obst) == 256
+    else:
+        g = np.arange(12) * 0.0165
+        cen, obst = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3), []
+    n = len(cen)
+    scene = particle_cloud_scene(cen, np.full(n, 0.0100), np.full(n, 20), obst, seed=4)
+    vel = np.zeros((scene["n_bodies"], 3))
+    vel[:n] = rng.uniform(-3.0, 3.0, (n, 3))
+    scene["vel"] = vel.reshape(-1).copy()
+    prm = StepParams.make(dt=1e-5, gravity=(0.0, -9.81, 0.0), spring=1e4, damper=0.1, friction=0.0)
+    stepped, graph, skin = _graph_and_stepped(ctx, scene, 8, 60, prm)
+    assert skin["rebuilds"] >= 2, skin
+    if kind == "dense":
+        assert 16384 < skin["capacity"] <= 32768, skin
+    _assert_same_run(stepped, graph)
+
+
+def test_graph_calls_of_every_length_equal_stepping(ctx, scene):
+    """Replays go out in graphs of 8 steps and of 1: calls of 1 to 17 steps in a row, contacts
+    carried from call to call, equal single steps."""
+    from delta_b200.engine import Simulation, StepParams
+
+    prm = StepParams.make(**PARAMS)
+    runs = []
+    for graph in (False, True):
+        sim = Simulation(ctx, scene, 8)
+        cps = [sim.step(k, prm, graph=graph) for k in (1, 7, 8, 9, 2, 16, 17)]
+        runs.append((np.concatenate(cps), sim.state(), sim.contacts(), sim.counters()))
+        sim.close()
+    (c0, s0, k0, n0), (c1, s1, k1, n1) = runs
+    assert np.array_equal(c0, c1) and n0 == n1
+    for k in STATE:
+        assert np.array_equal(s1[k], s0[k]), k
+    for f in FIELDS:
+        assert np.array_equal(k1[f], k0[f]), f
