@@ -812,62 +812,83 @@ __global__ void k_bucket_contacts(RawContacts rc, const uint32_t *poff, int64_t 
   bkey[j] = key;
 }
 
-// Step 2, one thread per bucket entry j of pair k (its key's): its rank is the number of
-// smaller keys in the pair's bucket (keys within a pair are distinct), and the contact is
-// written at poff[k] + rank, so the output is in (pair, A triangle, B triangle) order, the
-// order of a stable sort of all keys.  Thread 0 publishes the count and flags an overflow.
-// The block's keys and the 128 on either side are staged in shared memory: the ranks of the
-// buckets that lie within read nothing else.  (With a binary search of poff for the pair
-// and the bucket's keys read from memory one after another: 11 us of a hopper or box step.)
-constexpr int kGatherThreads = 256, kGatherHalo = 128;
+// Step 2, four threads per bucket entry j of pair k (its key's): its rank is the number of
+// smaller keys in the pair's bucket (keys within a pair are distinct), each thread counting
+// a quarter, and the contact is written at poff[k] + rank, a quarter of its fields each, so
+// the output is in (pair, A triangle, B triangle) order, the order of a stable sort of all
+// keys.  Thread 0 publishes the count and flags an overflow.
+// The keys of a block's 64 entries' pairs are staged in shared memory (their low words: the
+// triangle indices, which tell contacts of a pair apart); buckets that reach past the stage
+// are read from memory.  A step's few thousand contacts fill few SMs, and each waits for
+// its scattered sectors: a thread per entry, with a binary search of poff for the pair, took
+// 11 us of a hopper or box step (9 without the search).
+constexpr int kGatherThreads = 256, kGatherEntries = kGatherThreads / 4, kGatherKeys = 2048;
 __global__ void __launch_bounds__(kGatherThreads)
     k_pair_gather(RawContacts rc, const uint32_t *poff, const int64_t *bidx, const uint64_t *bkey, int64_t n_pairs,
                   delta_contacts out, int64_t *n_out, int *ovf, int ovf_code, int64_t *count_log) {
   dep_sync();
-  __shared__ uint64_t keys[kGatherThreads + 2 * kGatherHalo];
-  const int64_t blk0 = (int64_t)blockIdx.x * kGatherThreads, j = blk0 + threadIdx.x;
+  __shared__ uint32_t keys[kGatherKeys];
+  __shared__ uint32_t range[2];
+  const int e = threadIdx.x >> 2, part = threadIdx.x & 3;
+  const int64_t blk0 = (int64_t)blockIdx.x * kGatherEntries, j = blk0 + e;
   const unsigned long long cnt = *rc.count;
-  if (j == 0) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     const int64_t n = (int64_t)cnt < out.capacity ? (int64_t)cnt : out.capacity;
     *n_out = n;
     if (count_log) *count_log = n;
     if ((int64_t)cnt > out.capacity) atomicCAS(ovf, 0, ovf_code);
   }
-  const int64_t total = poff[n_pairs], lo = blk0 - kGatherHalo, hi = blk0 + kGatherThreads + kGatherHalo;
+  const uint32_t total = poff[n_pairs];
   if (blk0 >= total) return;
-  for (int t = threadIdx.x; t < kGatherThreads + 2 * kGatherHalo; t += kGatherThreads)
-    if (lo + t >= 0 && lo + t < total) keys[t] = bkey[lo + t];
+  const bool live = j < total;
+  const uint32_t low = (uint32_t)((1ull << (2 * rc.tbits)) - 1ull);
+  uint32_t base = 0, end = 0, own = 0;
+  int64_t s = 0;
+  if (live) {
+    const uint64_t key = bkey[j];
+    const int64_t k = (int64_t)(key >> (2 * rc.tbits));
+    base = poff[k];
+    end = poff[k + 1];
+    own = (uint32_t)key & low;
+    s = bidx[j];
+    if (threadIdx.x == 0) range[0] = base;
+    if (part == 0 && (j + 1 == total || e == kGatherEntries - 1)) range[1] = end;
+  }
   __syncthreads();
-  if (j >= total) return;
-  const uint64_t key = keys[threadIdx.x + kGatherHalo];
-  const int64_t k = (int64_t)(key >> (2 * rc.tbits)), base = poff[k], m = poff[k + 1] - base;
-  const int64_t s = bidx[j], cap = rc.cap, oc = out.capacity;
+  const uint32_t lo = range[0], hi = min(range[1], lo + kGatherKeys);
+  for (uint32_t t = lo + threadIdx.x; t < hi; t += kGatherThreads) keys[t - lo] = (uint32_t)bkey[t] & low;
+  __syncthreads();
   int rank = 0;
-  if (base >= lo && base + m <= hi) {
-    const uint64_t *b = keys + (base - lo);
-#pragma unroll 8
-    for (int i = 0; i < (int)m; ++i) rank += b[i] < key ? 1 : 0;
+  if (end <= hi) {
+#pragma unroll 4
+    for (uint32_t i = base + part; i < end; i += 4) rank += keys[i - lo] < own ? 1 : 0;
   } else {
-#pragma unroll 8
-    for (int64_t i = 0; i < m; ++i) rank += bkey[base + i] < key ? 1 : 0;
+#pragma unroll 4
+    for (uint32_t i = base + part; i < end; i += 4) rank += ((uint32_t)bkey[i] & low) < own ? 1 : 0;
   }
-  const int64_t d = base + rank;
-  if (d >= oc) return;
+  __syncwarp();
+  rank += __shfl_xor_sync(kFull, rank, 1);
+  rank += __shfl_xor_sync(kFull, rank, 2);
+  const int64_t d = (int64_t)base + rank, cap = rc.cap, oc = out.capacity;
+  if (!live || d >= oc) return;
+  // planes of rc.f: x, normal, depth, P, Q, eps_total
+  double *const dst = part == 0 ? out.x : part == 1 ? out.normal : part == 2 ? out.P : out.Q;
+  const int plane = part == 0 ? 0 : part == 1 ? 3 : part == 2 ? 7 : 10;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    out.x[k * oc + d] = rc.f[(0 + k) * cap + s];
-    out.normal[k * oc + d] = rc.f[(3 + k) * cap + s];
-    out.P[k * oc + d] = rc.f[(7 + k) * cap + s];
-    out.Q[k * oc + d] = rc.f[(10 + k) * cap + s];
+  for (int k = 0; k < 3; ++k) dst[k * oc + d] = rc.f[(plane + k) * cap + s];
+  if (part == 0) {
+    out.depth[d] = rc.f[6 * cap + s];
+    out.penetration[d] = 1;
+  } else if (part == 1) {
+    out.eps_total[d] = rc.f[13 * cap + s];
+    out.friction[d] = rc.fric[s];
+  } else if (part == 2) {
+    out.master[d] = rc.i[s];
+    out.slave[d] = rc.i[cap + s];
+  } else {
+    out.tri_a[d] = rc.i[2 * cap + s];
+    out.tri_b[d] = rc.i[3 * cap + s];
   }
-  out.depth[d] = rc.f[6 * cap + s];
-  out.eps_total[d] = rc.f[13 * cap + s];
-  out.master[d] = rc.i[s];
-  out.slave[d] = rc.i[cap + s];
-  out.tri_a[d] = rc.i[2 * cap + s];
-  out.tri_b[d] = rc.i[3 * cap + s];
-  out.penetration[d] = 1;
-  out.friction[d] = rc.fric[s];
 }
 
 __global__ void k_accumulate(const DevStats *st, int64_t *counters) {
@@ -1273,7 +1294,8 @@ delta_status detect_run_fixed(delta_ctx *ctx, cudaStream_t s, int driver, const 
     const unsigned cb = (unsigned)((cap + 255) / 256);
     if ((e = launch_dep(true, k_bucket_contacts, cb, 256, 0, s, rc, poff, perm_out, (uint64_t *)perm_in)) !=
             cudaSuccess ||
-        (e = launch_dep(true, k_pair_gather, cb, kGatherThreads, 0, s, rc, poff, perm_out, (const uint64_t *)perm_in,
+        (e = launch_dep(true, k_pair_gather, (unsigned)((cap + kGatherEntries - 1) / kGatherEntries), kGatherThreads, 0, s,
+                        rc, poff, perm_out, (const uint64_t *)perm_in,
                         pair_cap, out, d_ncontacts, d_ovf, ovf_code, d_count_log)) != cudaSuccess ||
         (e = launch_dep(true, k_cert_tail, 1, 1, 0, s, rc.sv_count, rc.sv_cap, dstats, d_ovf, d_counters, queue, end)) !=
             cudaSuccess)
