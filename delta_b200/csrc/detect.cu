@@ -1145,10 +1145,9 @@ delta_status detect_run(delta_ctx *ctx, int driver, int precision, const delta_m
   cudaStream_t s = ctx->stream;
   delta_status st;
   cudaError_t e;
-  void *small = nullptr, *pin = nullptr;
+  void *small = nullptr;
   if ((st = ctx_scratch(ctx, 5, sizeof(DetectSmall), &small)) != DELTA_OK) return st;
-  if ((st = ctx_pinned(ctx, sizeof(DetectSmall), &pin)) != DELTA_OK) return st;
-  DetectSmall *dev = (DetectSmall *)small, *host = (DetectSmall *)pin;
+  DetectSmall *dev = (DetectSmall *)small, back, *host = &back;
   // raw contact buffer: at least the caller's capacity; grown and rerun when it overflows
   const int64_t cap = out->capacity > 1024 ? out->capacity : 1024;
   RawContacts rc{};

@@ -2866,12 +2866,12 @@ delta_status delta_sim_step_graph(delta_sim *s, const delta_step_params *params,
   if ((e = cudaEventRecord(g.ev, s->ctx->stream)) != cudaSuccess ||
       (e = cudaStreamWaitEvent(g.stream, g.ev, 0)) != cudaSuccess)
     return cuda_error(e, "graph order");
-  void *pin = nullptr;
-  const size_t back_bytes = 256 + sizeof(int64_t) * (size_t)nsteps;
-  if ((ds = ctx_pinned(s->ctx, back_bytes, &pin)) != DELTA_OK) return ds;
+  // (plain host memory: pinning it cost a new simulation's first call 3 ms, and the copies
+  // are of a few hundred bytes that the host waits for anyway)
+  std::vector<int64_t> back((256 + sizeof(int64_t) * (size_t)nsteps) / sizeof(int64_t));
   if ((ds = copy_contacts(s->c, g.c, s->n_contacts, nullptr, g.stream)) != DELTA_OK) return ds;
   s->ctx->launches += 1;
-  GraphState *host = (GraphState *)pin;
+  GraphState *const host = (GraphState *)back.data();
   *host = GraphState{};
   host->n_contacts = s->n_contacts;
   host->need = -1;
@@ -2894,10 +2894,8 @@ delta_status delta_sim_step_graph(delta_sim *s, const delta_step_params *params,
         (ds = sim_all_vertices(s, g.stream)) != DELTA_OK)
       return ds;
     s->ctx->launches += 1;
-    if ((ds = ctx_pinned(s->ctx, back_bytes, &pin)) != DELTA_OK) return ds;
-    host = (GraphState *)pin;
-    const int64_t *log = (const int64_t *)((const char *)pin + 256);
-    if ((e = cudaMemcpyAsync(pin, g.dev, 256 + sizeof(int64_t) * (size_t)batch, cudaMemcpyDeviceToHost, g.stream)) !=
+    const int64_t *log = back.data() + 256 / sizeof(int64_t);
+    if ((e = cudaMemcpyAsync(back.data(), g.dev, 256 + sizeof(int64_t) * (size_t)batch, cudaMemcpyDeviceToHost, g.stream)) !=
             cudaSuccess ||
         (e = cudaStreamSynchronize(g.stream)) != cudaSuccess)
       return cuda_error(e, "graph sync");
