@@ -22,6 +22,13 @@
 //    between the families), and the closest points are computed from the winner in FP64.
 // Every feature attaining the reference minimum is a candidate, so the output equals
 // bfSolver's bit for bit.
+//
+// Bound by instruction issue (69%; 3290 a warp of 32 pairs).  What the FP64 side doesn't need
+// in FP64 is kept out of it: the extent and the candidates' comparison are in FP32 and the
+// winner's points are read from the staged coordinates by offset (they were loaded whole and
+// selected in registers).  4 M pairs 661 -> 577 us.  Tried: phases 2 and 3 as one loop over
+// the queue, for a single copy of the FP64 code in the instruction cache: 650 us; 80 registers
+// for six blocks an SM: no change; 72 for seven: 600 us.
 #pragma once
 #include "tri_ref.cuh"
 
@@ -152,74 +159,14 @@ __device__ __forceinline__ void pick_vertex(const R T[3][3], int i, R out[3]) {
   for (int k = 0; k < 3; ++k) out[k] = i == 0 ? T[0][k] : (i == 1 ? T[1][k] : T[2][k]);
 }
 
-// Reference value of feature f (runtime index) with one code path per family:
-// f < 9: edge-edge (eA = f/3, eB = f%3); else vertex-face j = f-9.
-__device__ __forceinline__ xf64 feature_dyn(const xf64 A[3][3], const xf64 B[3][3], int f, xf64 &p0, xf64 &p1) {
-  if (f < 9) {
-    const int ea = f / 3, eb = f - 3 * ea;
-    xf64 HA[3], TA[3], HB[3], TB[3];
-    pick_vertex(A, ea, HA);
-    pick_vertex(A, ea == 2 ? 0 : ea + 1, TA);
-    pick_vertex(B, eb, HB);
-    pick_vertex(B, eb == 2 ? 0 : eb + 1, TB);
-    return seg_seg_ref(HA, TA, HB, TB, p0, p1);
-  }
-  const int j = f - 9;
-  const bool onA = j < 3;
-  xf64 V0[3], V1[3], V2[3], X[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    V0[k] = onA ? A[0][k] : B[0][k];
-    V1[k] = onA ? A[1][k] : B[1][k];
-    V2[k] = onA ? A[2][k] : B[2][k];
-  }
-  const int xi = onA ? j : j - 3;
-  if (onA) pick_vertex(B, xi, X);
-  else pick_vertex(A, xi, X);
-  return pt_tri_ref(V0, V1, V2, X, p0, p1);
-}
-
-// Closest points of the winning feature (runtime index), bf.cpp:715-879 and 1104-1177.
-__device__ __forceinline__ void feature_points_dyn(const xf64 A[3][3], const xf64 B[3][3], int f, xf64 p0, xf64 p1,
-                                                   double pq[6]) {
-  if (f < 9) {
-    const int ea = f / 3, eb = f - 3 * ea;
-    xf64 HA[3], TA[3], HB[3], TB[3];
-    pick_vertex(A, ea, HA);
-    pick_vertex(A, ea == 2 ? 0 : ea + 1, TA);
-    pick_vertex(B, eb, HB);
-    pick_vertex(B, eb == 2 ? 0 : eb + 1, TB);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      pq[k] = (TA[k] + ((HA[k] - TA[k]) * p0)).v;
-      pq[3 + k] = (TB[k] + ((HB[k] - TB[k]) * p1)).v;
-    }
-    return;
-  }
-  const int j = f - 9;
-  const bool onA = j < 3;
-  xf64 X[3], face[3];
-  if (onA) pick_vertex(B, j, X);
-  else pick_vertex(A, j - 3, X);
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const xf64 v0 = onA ? A[0][k] : B[0][k], v1 = onA ? A[1][k] : B[1][k], v2 = onA ? A[2][k] : B[2][k];
-    face[k] = v0 + ((v2 - v0) * p1) + ((v1 - v0) * p0);
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    pq[k] = onA ? face[k].v : X[k].v;
-    pq[3 + k] = onA ? X[k].v : face[k].v;
-  }
-}
-
 // Per-warp shared staging for bf_cert_warp: the 32 pairs' FP64 coordinates, the
-// candidate queues (one per feature family) and the queue results.
+// candidate queues (one per feature family; entries lane << 4 | feature) and the queue
+// results.  A pair's row is 19 long: with an odd stride the lanes' 64-bit accesses to one
+// column of 16 rows fall on 16 different bank pairs (with 18, on 8).
 constexpr int kCertQueue = 64;  // entries evaluated per pass and family
 struct CertWarpSmem {
-  double coords[32][18];
-  uint8_t qs[32 * 9], qp[32 * 6];      // queued (lane << 0) with features in a separate array
-  uint8_t fs[32 * 9], fp[32 * 6];
+  double coords[32][19];
+  uint16_t qs[32 * 9], qp[32 * 6];
   double rd[kCertQueue], r0[kCertQueue], r1[kCertQueue];
   int32_t surv[64];  // particle-pair driver: B triangles that passed the box test
 };
@@ -233,16 +180,6 @@ struct FamilyBest {
     if (d < dist || (d == dist && ff < f)) { dist = d; f = ff; p0 = a; p1 = b; }
   }
 };
-
-__device__ __forceinline__ void load_pair(const CertWarpSmem &sm, int lane, xf64 A[3][3], xf64 B[3][3]) {
-#pragma unroll
-  for (int v = 0; v < 3; ++v)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      A[v][k] = xf64(sm.coords[lane][3 * v + k]);
-      B[v][k] = xf64(sm.coords[lane][9 + 3 * v + k]);
-    }
-}
 
 // Edge-edge feature f (0..8) of the pair staged for `lane`.
 __device__ __forceinline__ xf64 seg_dyn(const CertWarpSmem &sm, int lane, int f, xf64 &p0, xf64 &p1) {
@@ -273,17 +210,46 @@ __device__ __forceinline__ xf64 pt_dyn(const CertWarpSmem &sm, int lane, int j, 
   return pt_tri_ref(V0, V1, V2, X, p0, p1);
 }
 
+// Closest points of edge-edge feature f, bf.cpp:715-879.
+__device__ __forceinline__ void seg_points_dyn(const CertWarpSmem &sm, int lane, int f, xf64 p0, xf64 p1,
+                                               double pq[6]) {
+  const int ea = f / 3, eb = f - 3 * ea;
+  const int ta = ea == 2 ? 0 : ea + 1, tb = eb == 2 ? 0 : eb + 1;
+  const double *row = sm.coords[lane];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const xf64 HA(row[3 * ea + k]), TA(row[3 * ta + k]), HB(row[9 + 3 * eb + k]), TB(row[9 + 3 * tb + k]);
+    pq[k] = (TA + ((HA - TA) * p0)).v;
+    pq[3 + k] = (TB + ((HB - TB) * p1)).v;
+  }
+}
+
+// Closest points of vertex-face feature j, bf.cpp:1104-1177.
+__device__ __forceinline__ void pt_points_dyn(const CertWarpSmem &sm, int lane, int j, xf64 p0, xf64 p1,
+                                              double pq[6]) {
+  const bool onA = j < 3;
+  const double *tri = sm.coords[lane] + (onA ? 0 : 9), *pnt = sm.coords[lane] + (onA ? 9 + 3 * j : 3 * (j - 3));
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const xf64 v0(tri[k]), v1(tri[3 + k]), v2(tri[6 + k]), X(pnt[k]);
+    const xf64 face = v0 + ((v2 - v0) * p1) + ((v1 - v0) * p0);
+    pq[k] = onA ? face.v : X.v;
+    pq[3 + k] = onA ? X.v : face.v;
+  }
+}
+
 // Evaluates a family's queue (entries: lane, feature) in passes of kCertQueue and offers
 // each result to its owner's running minimum.  owner_lo/owner_cnt: this lane's entries.
 template <bool SEG>
-__device__ __forceinline__ void run_queue(CertWarpSmem &sm, const uint8_t *ql, const uint8_t *qf, int total,
-                                          int my_lo, int my_cnt, FamilyBest &best) {
+__device__ __forceinline__ void run_queue(CertWarpSmem &sm, const uint16_t *queue, int total, int my_lo, int my_cnt,
+                                          FamilyBest &best) {
   const int lane = threadIdx.x & 31;
   for (int base = 0; base < total; base += kCertQueue) {
     const int n = min(kCertQueue, total - base);
     for (int j = lane; j < n; j += 32) {
       xf64 p0, p1;
-      const xf64 d = SEG ? seg_dyn(sm, ql[base + j], qf[base + j], p0, p1) : pt_dyn(sm, ql[base + j], qf[base + j], p0, p1);
+      const int entry = queue[base + j];
+      const xf64 d = SEG ? seg_dyn(sm, entry >> 4, entry & 15, p0, p1) : pt_dyn(sm, entry >> 4, entry & 15, p0, p1);
       sm.rd[j] = d.v;
       sm.r0[j] = p0.v;
       sm.r1[j] = p1.v;
@@ -291,7 +257,7 @@ __device__ __forceinline__ void run_queue(CertWarpSmem &sm, const uint8_t *ql, c
     __syncwarp();
     const int lo = max(my_lo, base), hi = min(my_lo + my_cnt, base + n);
     for (int j = lo; j < hi; ++j)
-      best.offer(xf64(sm.rd[j - base]), qf[j], xf64(sm.r0[j - base]), xf64(sm.r1[j - base]));
+      best.offer(xf64(sm.rd[j - base]), queue[j] & 15, xf64(sm.r0[j - base]), xf64(sm.r1[j - base]));
     __syncwarp();
   }
 }
@@ -323,20 +289,20 @@ __device__ __forceinline__ int bf_cert_warp(const double A64[3][3], const double
     }
   // ---- 1. FP32 lower bounds -------------------------------------------------------
   float A[3][3], B[3][3];
-  double L = 0.0;
+  float L = 0.f;  // within 3 u32 L of the extent in FP64
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    double lo = A64[0][k], hi = A64[0][k];
+    float lo = 0.f, hi = 0.f;
 #pragma unroll
     for (int v = 0; v < 3; ++v) {
       A[v][k] = v == 0 ? 0.f : (float)(A64[v][k] - A64[0][k]);  // A's vertex 0 is the origin
       B[v][k] = (float)(B64[v][k] - A64[0][k]);
-      lo = fmin(lo, fmin(A64[v][k], B64[v][k]));
-      hi = fmax(hi, fmax(A64[v][k], B64[v][k]));
+      lo = fminf(lo, fminf(A[v][k], B[v][k]));
+      hi = fmaxf(hi, fmaxf(A[v][k], B[v][k]));
     }
-    L = fmax(L, hi - lo);
+    L = fmaxf(L, hi - lo);
   }
-  const float eps = (float)L * (64.f * kU32);
+  const float eps = L * (64.f * kU32);
   float lb[15];
   int sbest = 0, pbest = 0;
   float sd = 3.0e38f, pd = 3.0e38f;
@@ -378,34 +344,34 @@ __device__ __forceinline__ int bf_cert_warp(const double A64[3][3], const double
     if (dp < pt.dist) { pt.dist = dp; pt.f = pbest; pt.p0 = a0; pt.p1 = a1; }
   }
   const double best = fmin(seg.dist.v, pt.dist.v);  // NaN-free unless both are NaN
-  const double bound = (best == best) ? best : 1.0e308;
+  // (a float exceeds a double exactly when it exceeds the double rounded down)
+  const float bound = __double2float_rd((best == best) ? best : 1.0e308);
   // ---- 3. queue the remaining candidates, one queue per family ------------------------
   unsigned ms = 0, mp = 0;
 #pragma unroll
   for (int f = 0; f < 9; ++f)
-    if (f != sbest && !((double)lb[f] > bound)) ms |= 1u << f;
+    if (f != sbest && !(lb[f] > bound)) ms |= 1u << f;
 #pragma unroll
   for (int j = 0; j < 6; ++j)
-    if (j != pbest && !((double)lb[9 + j] > bound)) mp |= 1u << j;
+    if (j != pbest && !(lb[9 + j] > bound)) mp |= 1u << j;
   if (!valid) ms = mp = 0;
-  int ts, tp;
+  // both families' queue offsets from one scan (at most 9 * 32 and 6 * 32 entries)
   const int cs = __popc(ms), cp = __popc(mp);
-  const int os = warp_excl_scan(cs, ts), op = warp_excl_scan(cp, tp);
+  int both;
+  const int off = warp_excl_scan(cs | (cp << 16), both);
+  const int ts = both & 0xffff, tp = both >> 16, os = off & 0xffff, op = off >> 16;
   {
     int q = os;
-    for (unsigned m = ms; m; m &= m - 1) { sm.qs[q] = (uint8_t)lane; sm.fs[q] = (uint8_t)(__ffs(m) - 1); ++q; }
+    for (unsigned m = ms; m; m &= m - 1) sm.qs[q++] = (uint16_t)((lane << 4) | (__ffs(m) - 1));
     q = op;
-    for (unsigned m = mp; m; m &= m - 1) { sm.qp[q] = (uint8_t)lane; sm.fp[q] = (uint8_t)(__ffs(m) - 1); ++q; }
+    for (unsigned m = mp; m; m &= m - 1) sm.qp[q++] = (uint16_t)((lane << 4) | (__ffs(m) - 1));
   }
   __syncwarp();
-  run_queue<true>(sm, sm.qs, sm.fs, ts, os, cs, seg);
-  run_queue<false>(sm, sm.qp, sm.fp, tp, op, cp, pt);
+  run_queue<true>(sm, sm.qs, ts, os, cs, seg);
+  run_queue<false>(sm, sm.qp, tp, op, cp, pt);
   // ---- 4. selection (bf.cpp:1102) and closest points --------------------------------
-  xf64 Ax[3][3], Bx[3][3];
-  load_pair(sm, lane, Ax, Bx);
-  __syncwarp();
-  if (pt.dist > seg.dist) feature_points_dyn(Ax, Bx, seg.f, seg.p0, seg.p1, pq);
-  else feature_points_dyn(Ax, Bx, 9 + pt.f, pt.p0, pt.p1, pq);
+  if (pt.dist > seg.dist) seg_points_dyn(sm, lane, seg.f, seg.p0, seg.p1, pq);
+  else pt_points_dyn(sm, lane, pt.f, pt.p0, pt.p1, pq);
   return 2 + cs + cp;
 }
 
