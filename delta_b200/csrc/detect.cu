@@ -389,8 +389,15 @@ __global__ void __launch_bounds__(128, DetectBounds<R, DRV>::kMinBlocks) k_detec
 // lies in its body box and the per-axis gaps, their squares and their sum are monotone in
 // the boxes, so a triangle dropped against a body box fails against every triangle of
 // that body too.
+//
+// A step has fewer body pairs than the chip holds warps, so a pair's own chain of latencies
+// is what counts: the next pair is taken from the queue and its bodies are read while
+// this one is worked on, and survivors collect in shared memory (one atomic on the list's
+// counter per kCullBuffer / 2 of them or more, instead of one per group of lanes that found
+// some).
 constexpr int kCullThreads = 128;
-constexpr int kCullList = 256;
+constexpr int kCullList = 240;
+constexpr int kCullBuffer = 256;
 struct CullList {
   double lo[3][kCullList], hi[3][kCullList];
   uint16_t idx[kCullList];
@@ -465,42 +472,67 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
   dep_sync();
   __shared__ CullList LA, LB;
   __shared__ BodyPose QA, QB;
-  __shared__ int64_t s_next;
+  __shared__ double Alo[3], Ahi[3], Blo[3], Bhi[3];  // the bodies' boxes
+  __shared__ int64_t s_next[2];
+  __shared__ int2 s_bodies[2];
+  __shared__ uint64_t s_found[kCullBuffer];
+  __shared__ int s_nfound;
+  __shared__ int64_t s_base;
   const int tid = threadIdx.x;
   if (rc.pcnt && blockIdx.x == 0 && tid == 0) rc.pcnt[n_pairs] = 0;
+  if (tid == 0) s_nfound = 0;
+  // the block's survivors to the list (called by the whole block, after a barrier)
+  auto flush = [&]() {
+    const int n = s_nfound < kCullBuffer ? s_nfound : kCullBuffer;
+    if (tid == 0) s_base = (int64_t)atomicAdd(rc.sv_count, (unsigned long long)n);
+    __syncthreads();
+    for (int e = tid; e < n; e += kCullThreads)
+      if (s_base + e < rc.sv_cap) rc.sv[s_base + e] = s_found[e];
+    if (tid == 0) s_nfound = 0;
+  };
   // a persistent work queue of body pairs: each block takes the next pair when it is done
   // with its last, so uneven pairs (a wall of thousands of triangles next to small meshes)
-  // do not leave the other blocks idle; without a queue, a fixed stride
+  // do not leave the other blocks idle; without a queue, a fixed stride.  The first
+  // gridDim.x pairs go to the blocks by index.
   int64_t k = blockIdx.x;
-  if (rc.pair_queue) {
-    if (tid == 0) s_next = (int64_t)atomicAdd(rc.pair_queue, 1ull);
-    __syncthreads();
-    k = s_next;
+  int turn = 0;
+  int32_t a = 0, b = 0;
+  if (k < n_pairs) {
+    a = pa[k];
+    b = pb[k];
   }
   while (k < n_pairs) {
+    int64_t next = k + gridDim.x;  // thread 0's, if the pairs are queued
+    if (rc.pair_queue && tid == 0) next = (int64_t)gridDim.x + (int64_t)atomicAdd(rc.pair_queue, 1ull);
     do {  // one body pair; `continue` ends it
     if (rc.pcnt && tid == 0) rc.pcnt[k] = 0;  // the pair's contact count (k_cert_survivors)
-    const int32_t a = pa[k], b = pb[k];
     // (an index past the bodies is reported by k_check_detect)
     if (a < 0 || b < 0 || a >= m.n_bodies || b >= m.n_bodies) continue;
     const int64_t tA0 = m.tri_offset[a], tB0 = m.tri_offset[b];
     const int32_t nA = (int32_t)(m.tri_offset[a + 1] - tA0), nB = (int32_t)(m.tri_offset[b + 1] - tB0);
     if (tid == 0) atomicAdd(&st->tri_pairs, (unsigned long long)nA * (unsigned long long)nB);
     const double mg = (xf64(m.eps[a]) + xf64(m.eps[b])).v;
-    double Alo[3], Ahi[3], Blo[3], Bhi[3];
     const Pose &P = rc.pose;
-    if (P.rx) {
-      pose_box(P, a, Alo, Ahi);
-      pose_box(P, b, Blo, Bhi);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        Alo[c] = rc.bbox ? rc.bbox[6 * (int64_t)a + c] : -INFINITY;
-        Ahi[c] = rc.bbox ? rc.bbox[6 * (int64_t)a + 3 + c] : INFINITY;
-        Blo[c] = rc.bbox ? rc.bbox[6 * (int64_t)b + c] : -INFINITY;
-        Bhi[c] = rc.bbox ? rc.bbox[6 * (int64_t)b + 3 + c] : INFINITY;
+    const bool moveA = P.rx && !P.obstacle[a], moveB = P.rx && !P.obstacle[b];
+    // the bodies' boxes a thread per axis, their poses by the second warp
+    if (tid < 6) {
+      const int c = tid % 3;
+      const int32_t body = tid < 3 ? a : b;
+      double lo = -INFINITY, hi = INFINITY;
+      if (P.rx) {
+        pose_box_axis(P, body, c, lo, hi);
+      } else if (rc.bbox) {
+        lo = rc.bbox[6 * (int64_t)body + c];
+        hi = rc.bbox[6 * (int64_t)body + 3 + c];
       }
+      (tid < 3 ? Alo : Blo)[c] = lo;
+      (tid < 3 ? Ahi : Bhi)[c] = hi;
+    } else if (tid == 32) {
+      if (moveA) QA = body_pose(P, a);
+    } else if (tid == 33) {
+      if (moveB) QB = body_pose(P, b);
     }
+    __syncthreads();
     double cull = mg * (1.0 + 1e-9) + 1e-12;
     if (rc.rel_slack > 0.0) {
       double big = 0.0;
@@ -511,42 +543,61 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
     }
     const double cull2 = cull * cull;
     if (box_gap2(Alo, Ahi, Blo, Bhi) > cull2) continue;
-    const bool moveA = P.rx && !P.obstacle[a], moveB = P.rx && !P.obstacle[b];
-    if (tid == 0 && moveA) QA = body_pose(P, a);
-    if (tid == 1 && moveB) QB = body_pose(P, b);
-    __syncthreads();  // the poses are read by cull_fill (which synchronises before refilling)
     for (int32_t cb = 0; cb < nB;) {
       cb = cull_fill(m, P, moveB ? &QB : nullptr, tB0, nB, cb, Alo, Ahi, cull2, LB);
       const int nLB = LB.n;
       if (nLB == 0) continue;
       for (int32_t ca = 0; ca < nA;) {
         ca = cull_fill(m, P, moveA ? &QA : nullptr, tA0, nA, ca, Blo, Bhi, cull2, LA);
-        const int np = LA.n * nLB;
-        for (int j = tid; j < np; j += kCullThreads) {
-          const int ia = j / nLB, ib = j - ia * nLB;
+        const int nLA = LA.n, da = kCullThreads / nLB, db = kCullThreads - da * nLB;
+        for (int ia = tid / nLB, ib = tid - ia * nLB; ia < nLA;) {
           const double alo[3] = {LA.lo[0][ia], LA.lo[1][ia], LA.lo[2][ia]};
           const double ahi[3] = {LA.hi[0][ia], LA.hi[1][ia], LA.hi[2][ia]};
           const double blo[3] = {LB.lo[0][ib], LB.lo[1][ib], LB.lo[2][ib]};
           const double bhi[3] = {LB.hi[0][ib], LB.hi[1][ib], LB.hi[2][ib]};
           if (box_gap2(alo, ahi, blo, bhi) <= cull2) {
-            const int64_t pos = agg_slot(rc.sv_count);
-            if (pos < rc.sv_cap)
-              rc.sv[pos] = ((uint64_t)k << 32) | ((uint64_t)LA.idx[ia] << 16) | (uint64_t)LB.idx[ib];
+            const uint64_t key = ((uint64_t)k << 32) | ((uint64_t)LA.idx[ia] << 16) | (uint64_t)LB.idx[ib];
+            const int at = atomicAdd(&s_nfound, 1);
+            if (at < kCullBuffer) {
+              s_found[at] = key;
+            } else {
+              const int64_t pos = agg_slot(rc.sv_count);
+              if (pos < rc.sv_cap) rc.sv[pos] = key;
+            }
+          }
+          ia += da;  // the block's next 128 of the nLA * nLB pairs
+          ib += db;
+          if (ib >= nLB) {
+            ib -= nLB;
+            ++ia;
           }
         }
         __syncthreads();  // LA is refilled next
+        if (s_nfound > kCullBuffer / 2) flush();
       }
     }
     } while (0);
     if (rc.pair_queue) {
-      __syncthreads();  // every thread has read s_next for this pair
-      if (tid == 0) s_next = (int64_t)atomicAdd(rc.pair_queue, 1ull);
+      if (tid == 0) {
+        s_next[turn] = next;
+        s_bodies[turn] = next < n_pairs ? make_int2(pa[next], pb[next]) : make_int2(-1, -1);
+      }
       __syncthreads();
-      k = s_next;
+      next = s_next[turn];
+      a = s_bodies[turn].x;
+      b = s_bodies[turn].y;
+      turn ^= 1;
     } else {
-      k += gridDim.x;
+      if (next < n_pairs) {
+        a = pa[next];
+        b = pb[next];
+      }
+      __syncthreads();  // the boxes and poses have been read
     }
+    k = next;
   }
+  __syncthreads();
+  if (s_nfound > 0) flush();
 }
 
 // DELTA_CULL_STRIDE=1 in the environment: the culling kernel's blocks take the body pairs

@@ -97,30 +97,25 @@ __device__ __forceinline__ void posed_tri(const Pose &P, const BodyPose &q, int6
     posed_point(q.R, q.pos, q.rp, __ldg(P.rx + 3 * t + v), __ldg(P.ry + 3 * t + v), __ldg(P.rz + 3 * t + v), T[v]);
 }
 
-// A box (lo, hi) holding every current vertex of body b.  An obstacle has its stored box.
+// Axis k of a box (lo, hi) holding every current vertex of body b.  An obstacle has its
+// stored box.
 // A moving body's vertex is pos + R C with |C| <= reach, so along axis k it lies within
 // reach |row k of R| of pos_k (Cauchy-Schwarz); the half-width is widened by a relative
 // 1e-9 and by 1e-12 (|pos_k| + reach), far above the rounding of the vertex arithmetic
 // and of the bound itself.  A larger box only culls less, so the bound need not be tight.
-__device__ __forceinline__ void pose_box(const Pose &P, int32_t b, double lo[3], double hi[3]) {
+__device__ __forceinline__ void pose_box_axis(const Pose &P, int32_t b, int k, double &lo, double &hi) {
   if (P.obstacle[b]) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      lo[k] = P.obox[6 * (int64_t)b + k];
-      hi[k] = P.obox[6 * (int64_t)b + 3 + k];
-    }
+    lo = P.obox[6 * (int64_t)b + k];
+    hi = P.obox[6 * (int64_t)b + 3 + k];
     return;
   }
   const double reach = P.reach[b];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double r0 = P.rot[(int64_t)k * P.n + b], r1 = P.rot[(int64_t)(3 + k) * P.n + b],
-                 r2 = P.rot[(int64_t)(6 + k) * P.n + b];
-    const double c = P.pos[(int64_t)k * P.n + b];
-    const double h = reach * sqrt(r0 * r0 + r1 * r1 + r2 * r2) * (1.0 + 1e-9) + 1e-12 * (fabs(c) + reach);
-    lo[k] = c - h;
-    hi[k] = c + h;
-  }
+  const double r0 = P.rot[(int64_t)k * P.n + b], r1 = P.rot[(int64_t)(3 + k) * P.n + b],
+               r2 = P.rot[(int64_t)(6 + k) * P.n + b];
+  const double c = P.pos[(int64_t)k * P.n + b];
+  const double h = reach * sqrt(r0 * r0 + r1 * r1 + r2 * r2) * (1.0 + 1e-9) + 1e-12 * (fabs(c) + reach);
+  lo = c - h;
+  hi = c + h;
 }
 
 }  // namespace delta
