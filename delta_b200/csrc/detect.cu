@@ -43,7 +43,7 @@ struct RawContacts {
   // certified driver: per-body boxes (lo[3], hi[3]) for the culling, or null
   const double *bbox;
   // certified driver: with pose.rx set, the vertices are formed from the bodies' poses (the
-  // mesh arrays are not current) and the body boxes come from pose_box
+  // mesh arrays are not current) and the body boxes come from pose_box_axis
   Pose pose;
   // sort key of a contact: pair << 2 tbits | A triangle << tbits | B triangle
   int tbits;
@@ -468,7 +468,7 @@ __device__ __forceinline__ int32_t cull_fill(const delta_meshes &m, const Pose &
 // Pairs k = block, block + n_blocks, ... (entries with a negative body are empty).
 // Survivor keys (pair << 32 | A triangle << 16 | B triangle) go to rc.sv; their order is
 // free (the contacts are ordered by key afterwards).  With rc.pose the vertices are formed
-// from the bodies' poses and the body boxes come from pose_box; otherwise rc.bbox holds
+// from the bodies' poses and the body boxes from pose_box_axis; otherwise rc.bbox holds
 // the body boxes of the current vertices (null: no body-box tests).
 __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, const int32_t *__restrict__ pa,
                                                              const int32_t *__restrict__ pb, int64_t n_pairs,

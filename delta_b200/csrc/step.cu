@@ -1439,7 +1439,7 @@ static unsigned long long *broadphase_fixed_count(void *state, int32_t n) {
 // in the same order, as a grid search of that step.  A pair within reach now was within
 // reach + skin at the build if neither body has moved more than skin/2 since (triangle
 // inequality; the build test's relative and absolute margins cover the rounding), so the
-// list is rebuilt, inside the graph through a conditional node, in any step where some
+// list is rebuilt, inside the graph (k_skin_step, or a conditional node), in any step where some
 // moving body has moved further.  Obstacles do not move.
 struct SkinList {
   int64_t cap = 0;                          // entries of keys, raw, sel
