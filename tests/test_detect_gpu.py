@@ -192,3 +192,22 @@ def test_bf_driver_leaves_out_no_contact(ctx, oracle, kind):
     assert len(g) > 0
     for f in FIELDS:
         assert np.array_equal(g[f], o[f], equal_nan=True), f
+
+
+@pytest.mark.parametrize("sizes", [(1, 16), (15, 16), (16, 16), (17, 16), (120, 9), (241, 2), (2, 241), (300, 130)])
+@pytest.mark.parametrize("driver", [0, 8, 9])
+def test_culled_survivor_batches(ctx, oracle, driver, sizes):
+    """Every triangle pair survives the culling: batches of survivors below, at and above what
+    a block holds, and triangle lists longer than one window, give the serial loop's contacts
+    bit for bit."""
+    from delta_b200.detection import Meshes, detect
+
+    rng = np.random.default_rng(sizes[0] * 1000 + sizes[1])
+    bodies = [rng.uniform(-0.05, 0.05, (3, 3 * n)) for n in sizes + sizes[::-1]]
+    pa, pb = [0, 0, 1], [1, 3, 2]
+    eps_b, fric, ids = np.full(4, 0.2), np.zeros(4, np.uint8), np.arange(4)
+    g = detect(ctx, driver, Meshes.from_bodies(bodies, eps_b, fric, ids), pa, pb)[0].to_numpy()
+    o, _, _ = _oracle_contacts(oracle, 0, bodies, pa, pb, eps_b, fric, ids)
+    assert len(g) == len(o) == sum(bodies[a].shape[1] * bodies[b].shape[1] // 9 for a, b in zip(pa, pb))
+    for f in FIELDS:
+        assert np.array_equal(g[f], o[f], equal_nan=True), f

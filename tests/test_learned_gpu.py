@@ -463,3 +463,29 @@ def test_fused_train_step_vs_layer_path(ctx, pairs, M):
     import torch
 
     assert torch.equal(one.params_bf16, one.params.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("offset", [0.0, 1.0, 1e5, 1e8])
+def test_certified_pairs_hold_the_certificate_far_from_the_origin(ctx, offset):
+    """The certificate's rounding term grows with the largest coordinate: at every distance
+    from the origin the certified pairs satisfy it with the exact maximum, up to the rounding
+    of the two dot products (3 products and 2 sums of at most scale * d each: below 4e-15
+    scale * d together), and far enough out the term leaves close pairs uncertified."""
+    import torch
+
+    from delta_b200.learned import learned_pairs
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    n, tol = 20001, 1e-6
+    a = torch.rand((9, n), dtype=torch.float64, device="cuda", generator=g)
+    b = torch.rand((9, n), dtype=torch.float64, device="cuda", generator=g)
+    b[0::3] += 1.0 + 10.0 ** (-9.0 * torch.rand(n, dtype=torch.float64, device="cuda", generator=g))
+    a, b = (a + offset).contiguous(), (b + offset).contiguous()
+    p, q, d, fl = (t.cpu().numpy() for t in learned_pairs(ctx, None, a, b, sweeps=2, rel_tol=tol))
+    A, B, r = a.cpu().numpy().reshape(3, 3, n), b.cpu().numpy().reshape(3, 3, n), p - q
+    gap = np.einsum("vkn,kn->vn", A, r).min(0) - np.einsum("vkn,kn->vn", B, r).max(0)
+    scale = np.maximum(np.abs(A).max((0, 1)), np.abs(B).max((0, 1)))
+    ok = fl == 1
+    assert ok.any()
+    assert np.all((d * d - gap + 1e-14 * scale * d)[ok] <= (tol * d * d + 4e-15 * scale * d)[ok])
+    assert np.all(d[ok] * tol >= 0.6e-14 * scale[ok])
