@@ -57,6 +57,10 @@ struct RawContacts {
   unsigned long long *pair_queue;
   // culling distance added per unit of the largest coordinate of the two bodies' boxes
   double rel_slack;
+  // the caller's detections: result of the argument check (k_check_detect), launched before
+  // every kernel that follows a body's triangle range or a pair's bodies; those return at
+  // once when it is set.  Null: nothing to check
+  const int *bad;
 };
 
 struct DevStats {
@@ -296,8 +300,10 @@ __device__ void process_row(const delta_meshes &m, const RowCtx &r, const RawCon
   }
 }
 
-// per-body bounding boxes of the current vertices: one warp per body
-__global__ void k_body_boxes(delta_meshes m, double *__restrict__ bbox) {
+// per-body bounding boxes of the current vertices: one warp per body; none if the argument
+// check (*bad) failed, because the ranges it follows may then leave the vertex arrays
+__global__ void k_body_boxes(delta_meshes m, double *__restrict__ bbox, const int *__restrict__ bad) {
+  if (*bad) return;
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -474,6 +480,7 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
                                                              const int32_t *__restrict__ pb, int64_t n_pairs,
                                                              RawContacts rc, DevStats *st) {
   dep_sync();
+  if (rc.bad && *rc.bad) return;
   __shared__ CullList LA, LB;
   __shared__ BodyPose QA, QB;
   __shared__ double Alo[3], Ahi[3], Blo[3], Bhi[3];  // the bodies' boxes
@@ -510,8 +517,7 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
     if (rc.pair_queue && tid == 0) next = (int64_t)gridDim.x + (int64_t)atomicAdd(rc.pair_queue, 1ull);
     do {  // one body pair; `continue` ends it
     if (rc.pcnt && tid == 0) rc.pcnt[k] = 0;  // the pair's contact count (k_cert_survivors)
-    // (an index past the bodies is reported by k_check_detect)
-    if (a < 0 || b < 0 || a >= m.n_bodies || b >= m.n_bodies) continue;
+    if (a < 0 || b < 0) continue;
     const int64_t tA0 = m.tri_offset[a], tB0 = m.tri_offset[b];
     const int32_t nA = (int32_t)(m.tri_offset[a + 1] - tA0), nB = (int32_t)(m.tri_offset[b + 1] - tB0);
     if (tid == 0) atomicAdd(&st->tri_pairs, (unsigned long long)nA * (unsigned long long)nB);
@@ -1078,8 +1084,9 @@ static delta_status bad_argument(int bad) {
 }
 
 // The culled drivers' contacts into rc, unordered: argument check, box culling into the
-// survivor list, the survivors' solver, all enqueued at once (the solver reads the
-// survivors' number on the device); one read-back.  A buffer that was too small is grown
+// survivor list, the survivors' solver, all enqueued at once (after a failed check the
+// kernels that would read vertices return at once, and the solver finds no survivors; the
+// solver reads the survivors' number on the device); one read-back.  A buffer that was too small is grown
 // and the detection repeated.
 static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes &m, const int32_t *pa,
                                   const int32_t *pb, int64_t n_pairs, int64_t cap, DetectSmall *dev,
@@ -1090,17 +1097,16 @@ static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes
   if (!cull_stride()) rc.pair_queue = &dev->queue;
   rc.count = &dev->count;
   rc.sv_count = &dev->sv_count;
+  rc.bad = &dev->bad;
   if (pose) {
     rc.pose = *pose;  // current vertices and body boxes from the bodies' poses
   } else {
     // body boxes of the current vertices for the culling
     void *bb = nullptr;
     if ((st = ctx_scratch(ctx, 23, 48 * (size_t)m.n_bodies + 64, &bb)) != DELTA_OK) return st;
-    const int64_t warps = std::min<int64_t>(m.n_bodies, (int64_t)kNumSMs * 64);
-    k_body_boxes<<<(unsigned)std::max<int64_t>(1, (warps * 32 + 127) / 128), 128, 0, s>>>(m, (double *)bb);
-    ctx->launches += 1;
     rc.bbox = (const double *)bb;
   }
+  bool boxed = pose != nullptr;
   int64_t sv_cap = 8 * cap > (1 << 16) ? 8 * cap : (1 << 16);
   for (;;) {
     if ((st = raw_contacts(ctx, cap, rc)) != DELTA_OK) return st;
@@ -1112,6 +1118,13 @@ static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes
     const int64_t checks = std::max<int64_t>(n_pairs, m.n_bodies);
     k_check_detect<<<(unsigned)((checks + 255) / 256), 256, 0, s>>>(m.tri_offset, pa, pb, n_pairs, m.n_bodies,
                                                                    &dev->bad);
+    if (!boxed) {
+      const int64_t warps = std::min<int64_t>(m.n_bodies, (int64_t)kNumSMs * 64);
+      k_body_boxes<<<(unsigned)std::max<int64_t>(1, (warps * 32 + 127) / 128), 128, 0, s>>>(
+          m, const_cast<double *>(rc.bbox), rc.bad);
+      ctx->launches += 1;
+      boxed = true;
+    }
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_error(e, "detect check");
     if ((e = launch_cull(s, m, pa, pb, n_pairs, rc, &dev->stats, ctx->cull_blocks_per_sm)) != cudaSuccess)
       return cuda_error(e, "cull kernel");
