@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "tcphase.h"
 
 namespace delta {
 
@@ -181,7 +182,9 @@ delta_status delta_synchronize(delta_ctx *ctx) {
     return cuda_error(e, "gemm flag");
   if (!flag) return DELTA_OK;
   cudaMemset(ctx->gemm_err, 0, sizeof(int));
-  return set_error(DELTA_ERR_TIMEOUT, "tcgen05 GEMM: bounded wait for the tensor cores gave up");
+  return set_error(DELTA_ERR_TIMEOUT, flag == kTcLost
+                                          ? "tcgen05 GEMM: bounded wait for the tensor cores gave up, their work lost"
+                                          : "tcgen05 GEMM: bounded wait for the tensor cores gave up");
 }
 
 int64_t delta_launch_count(const delta_ctx *ctx) { return ctx ? ctx->launches : 0; }

@@ -506,9 +506,9 @@ __device__ __forceinline__ void group_sync(int g) { asm volatile("bar.sync %0, 1
 // everyone waits (at most `spin` polls).  Returns false (and sets the warpgroup's abort
 // flag) when the wait timed out.  `withhold` (the time-out test only) issues neither the
 // MMAs nor the commit, so the barrier never completes and the wait runs out with nothing in
-// flight.
+// flight.  (`phase` is the first thread's.)
 __device__ __forceinline__ bool tc_layer(TcSmem &sm, int g, uint32_t tmem, const __nv_bfloat16 *W, int K, int N,
-                                         uint32_t &phase, uint32_t spin, bool withhold = false) {
+                                         TcPhase &phase, uint32_t spin, bool withhold = false) {
   // make the generic-proxy stores of A visible to the tensor cores, then synchronise
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -522,10 +522,9 @@ __device__ __forceinline__ bool tc_layer(TcSmem &sm, int g, uint32_t tmem, const
         tc_mma(tmem, tc_desc(a0 + 256u * s, 16u * K), tc_desc(w0 + 256u * s, 16u * K), idesc, s > 0 ? 1u : 0u);
       tc_commit(&sm.mbar[g]);
     }
-    if (!tc_wait(&sm.mbar[g], phase, spin)) sm.abort[g] = 1;
+    if (!phase.wait([&](uint32_t parity) { return tc_wait(&sm.mbar[g], parity, spin); })) sm.abort[g] = 1;
   }
   group_sync(g);
-  phase ^= 1u;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   return sm.abort[g] == 0;
 }
@@ -569,7 +568,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   // this thread's TMEM lane (row) in bits 16..31 of the address, column in bits 0..15
   const uint32_t tlane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
   char *ah = reinterpret_cast<char *>(sm.ah[g]);
-  uint32_t phase = 0;
+  TcPhase phase;
   bool ok = true;
   const int64_t tiles = (n + kTcRows - 1) / kTcRows;
   // (the warpgroups of one SM take tiles a grid apart: short lists spread over the SMs)
@@ -621,12 +620,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                       v[3] + sm.bias[3 * kHid + 3]);
   }
   if (!ok && r == 0) {
-    // after a time-out: whatever was issued must end before the TMEM is freed (bounded)
-    if (!withhold) {
-      tc_commit(&sm.mbar[g]);
-      tc_wait(&sm.mbar[g], phase, spin);
-    }
-    atomicExch(err, 1);
+    // after a time-out: one more bounded wait for the commit that was late, so that nothing is
+    // in flight when the TMEM is freed (unless it runs out too, which the flag reports)
+    const bool drained =
+        withhold || phase.drain([&](uint32_t parity) { return tc_wait(&sm.mbar[g], parity, spin); });
+    atomicMax(err, drained ? kTcLate : kTcLost);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -868,7 +866,7 @@ __global__ void __launch_bounds__(kGtThreads) k_gemm_tc(int M, int N, int K, con
     }
     __syncwarp();
   }
-  if (!ok && tid == 0) atomicExch(err, 1);
+  if (!ok && tid == 0) atomicMax(err, kTcLate);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
@@ -1278,8 +1276,11 @@ delta_status mlp_check_error(delta_ctx *ctx, const int *err) {
   if ((e = cudaMemcpyAsync(pin, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||
       (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
     return cuda_error(e, "mlp status");
-  if (*static_cast<int *>(pin))
-    return set_error(DELTA_ERR_TIMEOUT, "tcgen05 inference: bounded wait for the tensor cores gave up");
+  const int flag = *static_cast<int *>(pin);
+  if (flag)
+    return set_error(DELTA_ERR_TIMEOUT, flag == kTcLost
+                                            ? "tcgen05 inference: bounded wait for the tensor cores gave up, their work lost"
+                                            : "tcgen05 inference: bounded wait for the tensor cores gave up");
   return DELTA_OK;
 }
 

@@ -5,6 +5,8 @@
 
 #include <cstdint>
 
+#include "tcphase.h"
+
 namespace delta {
 
 namespace {

@@ -106,10 +106,10 @@ __device__ __forceinline__ void tr_publish() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 // Waits (bounded) for everything thread 0 has issued and committed; false on time-out.
-__device__ __forceinline__ bool tr_wait(TrainSmem &sm, uint32_t &phase) {
-  if (threadIdx.x == 0 && !tc_wait(&sm.mbar, phase, kTcSpin)) sm.abort = 1;
+// (`phase` is thread 0's.)
+__device__ __forceinline__ bool tr_wait(TrainSmem &sm, TcPhase &phase) {
+  if (threadIdx.x == 0 && !phase.wait([&](uint32_t parity) { return tc_wait(&sm.mbar, parity, kTcSpin); })) sm.abort = 1;
   __syncthreads();
-  phase ^= 1u;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   return sm.abort == 0;
 }
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(kTrThreads, 1)
   const uint32_t tmem = sm.tmem_base;
   const int r = (warp & 3) * 32 + lane, part_c = warp >> 2, c0 = 32 * part_c;
   const uint32_t tlane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-  uint32_t phase = 0;
+  TcPhase phase;
   float db[3][8] = {}, dw1[8] = {}, dw4[4] = {}, db4[4] = {}, loss = 0.f;
   // the last tile's dW1 (8 columns a thread) and dW4 (threads of the first 4 warps)
   auto add_small = [&]() {
@@ -323,11 +323,19 @@ __global__ void __launch_bounds__(kTrThreads, 1)
     }
     column_sums(sm.dz, db[0]);
   }
-  // the last tile's products, also after a time-out: nothing may be in flight when the TMEM
-  // is freed
-  __syncthreads();
-  if (tid == 0) tc_commit(&sm.mbar);
-  if (!tr_wait(sm, phase)) ok = false;
+  // the last tile's products
+  if (ok) {
+    __syncthreads();
+    if (tid == 0) tc_commit(&sm.mbar);
+    ok = tr_wait(sm, phase);
+  }
+  // after a time-out thread 0 waits once more, bounded, for the commit that was late (it
+  // tracks every MMA issued before it): nothing is in flight when the TMEM is freed, unless
+  // that wait runs out too, which the flag reports
+  if (!ok && tid == 0) {
+    const bool drained = phase.drain([&](uint32_t parity) { return tc_wait(&sm.mbar, parity, kTcSpin); });
+    atomicMax(err, drained ? kTcLate : kTcLost);
+  }
   float *out = part + (int64_t)blockIdx.x * kPartStride;
   if (ok) {
     add_small();
@@ -380,7 +388,6 @@ __global__ void __launch_bounds__(kTrThreads, 1)
     }
   } else {
     for (int64_t e = tid; e < kPartStride; e += kTrThreads) out[e] = __int_as_float(0x7fc00000);
-    if (tid == 0) atomicExch(err, 1);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
