@@ -1,0 +1,70 @@
+"""Detections with many survivors of the box culling: every pair of long thin triangles that
+cross the same space has overlapping boxes, and few of them touch."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("x", "normal", "depth", "P", "Q", "eps_total", "master", "slave", "tri_a", "tri_b")
+
+
+def needles(triangles, seed):
+    """Vertices (3 * triangles, 3) of thin triangles, each across the unit cube."""
+    rng = np.random.default_rng(seed)
+    a = rng.uniform(0.0, 0.2, (triangles, 3))
+    b = rng.uniform(0.8, 1.0, (triangles, 3))
+    flip = rng.random((triangles, 3)) < 0.5  # along the four diagonals
+    a, b = np.where(flip, b, a), np.where(flip, a, b)
+    return np.stack([a, b, b + rng.uniform(-0.01, 0.01, (triangles, 3))], 1).reshape(-1, 3)
+
+
+def bodies(sizes, seed=0, eps=5e-6):
+    from delta_b200 import detection
+
+    xyz = np.concatenate([needles(n, seed + k) for k, n in enumerate(sizes)])
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    n = len(sizes)
+    return detection.Meshes(off, *(xyz[:, k].copy() for k in range(3)), np.full(n, eps), np.zeros(n, np.uint8))
+
+
+def detect(ctx, driver, meshes, pairs, contacts):
+    import torch
+
+    from delta_b200 import lib
+
+    pa, pb = (torch.tensor(p, dtype=torch.int32).cuda() for p in zip(*pairs))
+    count = ctypes.c_int64(0)
+    launches = lib().delta_launch_count(ctx.handle)
+    status = lib().delta_detect(ctx.handle, driver, 0, ctypes.byref(meshes.struct()), pa.data_ptr(), pb.data_ptr(),
+                                len(pairs), ctypes.byref(contacts.struct()), ctypes.byref(count), None)
+    assert status == 0, status
+    rows = contacts.to_numpy(count.value)
+    return rows, lib().delta_launch_count(ctx.handle) - launches
+
+
+@pytest.mark.parametrize("name", ["bf", "bf_cert", "bf_culled", "learned"])
+def test_a_long_survivor_list_is_kept_from_call_to_call(name):
+    """160,801 survivors do not fit a new context's list of 65,536: the first call culls twice,
+    the later ones launch each kernel once, and all return the contacts of a context whose list
+    was long enough from the start."""
+    from delta_b200 import detection
+    from delta_b200.narrowphase import Context
+
+    driver = {"bf": detection.DRV_BF, "bf_cert": detection.DRV_BF_CERT, "bf_culled": detection.DRV_BF_CULLED,
+              "learned": detection.DRV_LEARNED}[name]
+    sizes, pairs = [401] * 6, [(k, k + 1) for k in range(5)]  # 804,005 triangle pairs
+    m = bodies(sizes)
+    ctx = Context(0)
+    runs = [detect(ctx, driver, m, pairs, detection.Contacts(4096)) for _ in range(3)]
+    ctx.close()
+    long = Context(0)
+    want, least = detect(long, driver, m, pairs, detection.Contacts(1 << 17))
+    long.close()
+    assert 0 < len(want) <= 4096
+    for rows, _ in runs:
+        assert len(rows) == len(want)
+        for f in FIELDS:
+            assert np.array_equal(rows[f], want[f]), f
+    assert runs[0][1] > least and [n for _, n in runs[1:]] == [least, least]
