@@ -61,7 +61,39 @@ struct RawContacts {
   // every kernel that follows a body's triangle range or a pair's bodies; those return at
   // once when it is set.  Null: nothing to check
   const int *bad;
+  // bf()'s culling: the list's triangle pairs (k_check_detect), which its slices are cut by;
+  // null elsewhere
+  const struct PairWork *work;
 };
+
+// The triangle pairs of a list of body pairs: their number, the most in one pair, and the most
+// triangles of a second body.
+struct PairWork {
+  unsigned long long total, most;
+  unsigned long long most_b;
+};
+
+// Slices of the second body that bf()'s culling cuts every body pair into, each an item of
+// its queue.  One block to a pair leaves the chip idle where a few pairs of large bodies are
+// all there is (two bodies of 5,120 triangles, one half inside the other: 16.1 ms with one
+// block, 0.35 with slices, 6.8 with every triangle pair solved on the whole chip; of 20,480:
+// 253, 1.6 and 94 ms).  Slices of about 2^14 triangle pairs (with 2^15, 2^16, 2^17: a pair of
+// 320 x 320 with all surviving 233 us a call, 281, 417, 346; the others within 10%), not so
+// many that there are more than 16 a SM, nor of fewer than 32 triangles.
+constexpr int64_t kSlicePairs = 1 << 14, kSliceItems = 16 * kNumSMs;
+__host__ __device__ inline int64_t cull_slices(const PairWork &w, int64_t n_pairs) {
+  int64_t s = ((int64_t)w.most + kSlicePairs - 1) / kSlicePairs;
+  const int64_t fit = kSliceItems / n_pairs, b = ((int64_t)w.most_b + 31) / 32;
+  s = s < fit ? s : fit;
+  s = s < b ? s : b;
+  return s > 1 ? s : 1;
+}
+// bf()'s culling would wait for one block that works on one large pair while the others are
+// done: a block takes 0.7 to 5 ns a triangle pair (few survivors, all), the chip 0.22 ns to
+// solve one without culling.
+__host__ __device__ inline bool cull_uneven(const PairWork &w, int64_t n_pairs) {
+  return 8 * (w.most / (unsigned long long)cull_slices(w, n_pairs)) > w.total + (1ull << 19);
+}
 
 struct DevStats {
   unsigned long long hist[17];
@@ -475,12 +507,21 @@ __device__ __forceinline__ int32_t cull_fill(const delta_meshes &m, const Pose &
 // Survivor keys (pair << 32 | A triangle << 16 | B triangle) go to rc.sv; their order is
 // free (the contacts are ordered by key afterwards).  With rc.pose the vertices are formed
 // from the bodies' poses and the body boxes from pose_box_axis; otherwise rc.bbox holds
-// the body boxes of the current vertices (null: no body-box tests).
+// the body boxes of the current vertices (null: no body-box tests).  kSliced (bf()'s): the
+// items are slices of the pairs (cull_slices), item k slice k mod S of pair k / S.
+template <bool kSliced>
 __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, const int32_t *__restrict__ pa,
                                                              const int32_t *__restrict__ pb, int64_t n_pairs,
                                                              RawContacts rc, DevStats *st) {
   dep_sync();
   if (rc.bad && *rc.bad) return;
+  int64_t slices = 1;
+  if constexpr (kSliced) {
+    const PairWork work = *rc.work;
+    if (cull_uneven(work, n_pairs)) return;  // (the host solves every triangle pair)
+    slices = cull_slices(work, n_pairs);
+  }
+  const int64_t n_items = n_pairs * slices;
   __shared__ CullList LA, LB;
   __shared__ BodyPose QA, QB;
   __shared__ double Alo[3], Ahi[3], Blo[3], Bhi[3];  // the bodies' boxes
@@ -508,19 +549,28 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
   int64_t k = blockIdx.x;
   int turn = 0;
   int32_t a = 0, b = 0;
-  if (k < n_pairs) {
-    a = pa[k];
-    b = pb[k];
+  auto pair_of = [&](int64_t item) { return !kSliced || slices == 1 ? item : item / slices; };
+  if (k < n_items) {
+    a = pa[pair_of(k)];
+    b = pb[pair_of(k)];
   }
-  while (k < n_pairs) {
+  while (k < n_items) {
     int64_t next = k + gridDim.x;  // thread 0's, if the pairs are queued
     if (rc.pair_queue && tid == 0) next = (int64_t)gridDim.x + (int64_t)atomicAdd(rc.pair_queue, 1ull);
     do {  // one body pair; `continue` ends it
+    const int64_t pair = pair_of(k);
     if (rc.pcnt && tid == 0) rc.pcnt[k] = 0;  // the pair's contact count (k_cert_survivors)
     if (a < 0 || b < 0) continue;
     const int64_t tA0 = m.tri_offset[a], tB0 = m.tri_offset[b];
     const int32_t nA = (int32_t)(m.tri_offset[a + 1] - tA0), nB = (int32_t)(m.tri_offset[b + 1] - tB0);
-    if (tid == 0) atomicAdd(&st->tri_pairs, (unsigned long long)nA * (unsigned long long)nB);
+    int32_t b0 = 0, b1 = nB;  // this item's triangles of the second body
+    if (kSliced && slices > 1) {
+      const int32_t per = (int32_t)((nB + slices - 1) / slices), slice = (int32_t)(k - pair * slices);
+      b0 = per * slice;
+      b1 = b0 + per < nB ? b0 + per : nB;
+    }
+    if (tid == 0 && b0 == 0) atomicAdd(&st->tri_pairs, (unsigned long long)nA * (unsigned long long)nB);
+    if (kSliced && b0 >= b1) continue;
     const double mg = (xf64(m.eps[a]) + xf64(m.eps[b])).v;
     const Pose &P = rc.pose;
     const bool moveA = P.rx && !P.obstacle[a], moveB = P.rx && !P.obstacle[b];
@@ -553,8 +603,8 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
     }
     const double cull2 = cull * cull;
     if (box_gap2(Alo, Ahi, Blo, Bhi) > cull2) continue;
-    for (int32_t cb = 0; cb < nB;) {
-      cb = cull_fill(m, P, moveB ? &QB : nullptr, tB0, nB, cb, Alo, Ahi, cull2, LB);
+    for (int32_t cb = b0; cb < b1;) {
+      cb = cull_fill(m, P, moveB ? &QB : nullptr, tB0, b1, cb, Alo, Ahi, cull2, LB);
       const int nLB = LB.n;
       if (nLB == 0) continue;
       for (int32_t ca = 0; ca < nA;) {
@@ -566,7 +616,7 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
           const double blo[3] = {LB.lo[0][ib], LB.lo[1][ib], LB.lo[2][ib]};
           const double bhi[3] = {LB.hi[0][ib], LB.hi[1][ib], LB.hi[2][ib]};
           if (box_gap2(alo, ahi, blo, bhi) <= cull2) {
-            const uint64_t key = ((uint64_t)k << 32) | ((uint64_t)LA.idx[ia] << 16) | (uint64_t)LB.idx[ib];
+            const uint64_t key = ((uint64_t)pair << 32) | ((uint64_t)LA.idx[ia] << 16) | (uint64_t)LB.idx[ib];
             const int at = atomicAdd(&s_nfound, 1);
             if (at < kCullBuffer) {
               s_found[at] = key;
@@ -590,7 +640,7 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
     if (rc.pair_queue) {
       if (tid == 0) {
         s_next[turn] = next;
-        s_bodies[turn] = next < n_pairs ? make_int2(pa[next], pb[next]) : make_int2(-1, -1);
+        s_bodies[turn] = next < n_items ? make_int2(pa[pair_of(next)], pb[pair_of(next)]) : make_int2(-1, -1);
       }
       __syncthreads();
       next = s_next[turn];
@@ -598,9 +648,9 @@ __global__ void __launch_bounds__(kCullThreads, 8) k_cull_pairs(delta_meshes m, 
       b = s_bodies[turn].y;
       turn ^= 1;
     } else {
-      if (next < n_pairs) {
-        a = pa[next];
-        b = pb[next];
+      if (next < n_items) {
+        a = pa[pair_of(next)];
+        b = pb[pair_of(next)];
       }
       __syncthreads();  // the boxes and poses have been read
     }
@@ -624,12 +674,16 @@ inline bool cull_stride() {
 inline cudaError_t launch_cull(cudaStream_t s, const delta_meshes &m, const int32_t *pa, const int32_t *pb,
                                int64_t n_pairs, const RawContacts &rc, DevStats *st, int cap = 0, bool dep = false) {
   int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cull_pairs, kCullThreads, 0);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cull_pairs<false>, kCullThreads, 0);
   if (e != cudaSuccess) return e;
   if (cap > 0 && cap < per_sm) per_sm = cap;
   int64_t blocks = (int64_t)kNumSMs * (per_sm > 0 ? per_sm : 1);
+  if (rc.work) {  // (the number of slices is known on the device)
+    k_cull_pairs<true><<<(unsigned)blocks, kCullThreads, 0, s>>>(m, pa, pb, n_pairs, rc, st);
+    return cudaGetLastError();
+  }
   if (blocks > n_pairs) blocks = n_pairs > 0 ? n_pairs : 1;
-  return launch_dep(dep, k_cull_pairs, (unsigned)blocks, kCullThreads, 0, s, m, pa, pb, n_pairs, rc, st);
+  return launch_dep(dep, k_cull_pairs<false>, (unsigned)blocks, kCullThreads, 0, s, m, pa, pb, n_pairs, rc, st);
 }
 
 // The survivors to solve.  A caller's detection with more of them than the list holds is
@@ -805,14 +859,36 @@ inline cudaError_t launch_survivors(int driver, cudaStream_t s, const delta_mesh
 }
 
 // Argument check: bad = 1 for a body index out of range, else 2 for a
-// body of 65536 or more triangles.
+// body of 65536 or more triangles.  With `work`: the list's triangle pairs, if none is bad.
 __global__ void k_check_detect(const int64_t *tri_offset, const int32_t *pa, const int32_t *pb, int64_t n_pairs,
-                               int32_t n_bodies, int *bad) {
+                               int32_t n_bodies, int *bad, PairWork *work) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n_pairs && (pa[t] < 0 || pa[t] >= n_bodies || pb[t] < 0 || pb[t] >= n_bodies)) atomicExch(bad, 1);
+  unsigned long long pairs = 0, in_b = 0;
+  if (t < n_pairs) {
+    const int32_t a = pa[t], b = pb[t];
+    if (a < 0 || a >= n_bodies || b < 0 || b >= n_bodies) {
+      atomicExch(bad, 1);
+    } else if (work) {
+      in_b = (unsigned long long)(tri_offset[b + 1] - tri_offset[b]);
+      pairs = (unsigned long long)(tri_offset[a + 1] - tri_offset[a]) * in_b;
+    }
+  }
   if (t < n_bodies) {
     const int64_t n = tri_offset[t + 1] - tri_offset[t];
     if (n < 0 || n >= 65536) atomicCAS(bad, 0, 2);
+  }
+  if (!work) return;
+  unsigned long long most = pairs;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    pairs += __shfl_xor_sync(kFull, pairs, o);
+    most = max(most, __shfl_xor_sync(kFull, most, o));
+    in_b = max(in_b, __shfl_xor_sync(kFull, in_b, o));
+  }
+  if ((threadIdx.x & 31) == 0 && pairs) {
+    atomicAdd(&work->total, pairs);
+    atomicMax(&work->most, most);
+    atomicMax(&work->most_b, in_b);
   }
 }
 
@@ -1051,7 +1127,7 @@ cudaError_t launch_detect_prec(int driver, cudaStream_t s, const delta_meshes &m
 }  // namespace
 
 cudaError_t detect_launch_limits(int driver, int *cull_per_sm, int *surv_per_sm) {
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(cull_per_sm, k_cull_pairs, kCullThreads, 0);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(cull_per_sm, k_cull_pairs<false>, kCullThreads, 0);
   if (e != cudaSuccess) return e;
   return driver == DELTA_DRV_BF_CULLED
              ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(surv_per_sm, k_bf64_survivors, 128, 0)
@@ -1064,7 +1140,9 @@ cudaError_t detect_launch_limits(int driver, int *cull_per_sm, int *surv_per_sm)
 // work queue, the contact count and the survivor count.
 struct DetectSmall {
   int bad;
-  char pad[252];
+  char pad[4];
+  PairWork work;
+  char pad2[224];
   DevStats stats;
   unsigned long long queue, count, sv_count, unused[5];
 };
@@ -1092,10 +1170,11 @@ static delta_status bad_argument(int bad) {
 // survivor list, the survivors' solver, all enqueued at once (after a failed check the
 // kernels that would read vertices return at once, and the solver finds no survivors; the
 // solver reads the survivors' number on the device); one read-back.  A buffer that was too small is grown
-// and the detection repeated.
+// and the detection repeated.  With `rows` (bf()), *rows is set where the culling is not for
+// this list (cull_uneven) and nothing was detected.
 static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes &m, const int32_t *pa,
                                   const int32_t *pb, int64_t n_pairs, int64_t cap, DetectSmall *dev,
-                                  DetectSmall *host, const Pose *pose, RawContacts &rc) {
+                                  DetectSmall *host, const Pose *pose, RawContacts &rc, bool *rows) {
   cudaStream_t s = ctx->stream;
   delta_status st;
   cudaError_t e;
@@ -1103,6 +1182,7 @@ static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes
   rc.count = &dev->count;
   rc.sv_count = &dev->sv_count;
   rc.bad = &dev->bad;
+  if (rows) rc.work = &dev->work;
   if (pose) {
     rc.pose = *pose;  // current vertices and body boxes from the bodies' poses
   } else {
@@ -1126,7 +1206,7 @@ static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes
     if ((e = cudaMemsetAsync(dev, 0, sizeof(DetectSmall), s)) != cudaSuccess) return cuda_error(e, "detect memset");
     const int64_t checks = std::max<int64_t>(n_pairs, m.n_bodies);
     k_check_detect<<<(unsigned)((checks + 255) / 256), 256, 0, s>>>(m.tri_offset, pa, pb, n_pairs, m.n_bodies,
-                                                                   &dev->bad);
+                                                                   &dev->bad, rows ? &dev->work : nullptr);
     if (!boxed) {
       const int64_t warps = std::min<int64_t>(m.n_bodies, (int64_t)kNumSMs * 64);
       k_body_boxes<<<(unsigned)std::max<int64_t>(1, (warps * 32 + 127) / 128), 128, 0, s>>>(
@@ -1144,6 +1224,7 @@ static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
       return cuda_error(e, "detect counts");
     if (host->bad) return bad_argument(host->bad);
+    if (rows && (*rows = cull_uneven(host->work, n_pairs))) return DELTA_OK;
     host->stats.evaluated = host->sv_count;
     const int64_t nsv = (int64_t)host->sv_count, nc = (int64_t)host->count;
     if (nsv > sv_cap) sv_cap = nsv + nsv / 4;
@@ -1167,7 +1248,7 @@ static delta_status detect_rows(delta_ctx *ctx, int driver, int precision, const
   int64_t *rows = (int64_t *)rbuf, *row_offset = rows + n_pairs + 1;
   const int64_t checks = std::max<int64_t>(n_pairs, m.n_bodies);
   k_check_detect<<<(unsigned)((checks + 255) / 256), 256, 0, s>>>(m.tri_offset, pa, pb, n_pairs, m.n_bodies,
-                                                                 &dev->bad);
+                                                                 &dev->bad, nullptr);
   k_rows_per_pair<<<(unsigned)((n_pairs + 256) / 256), 256, 0, s>>>(m.tri_offset, pa, n_pairs, m.n_bodies, rows);
   ctx->launches += 2;
   size_t temp_bytes = 0;
@@ -1230,12 +1311,16 @@ delta_status detect_run(delta_ctx *ctx, int driver, int precision, const delta_m
   RawContacts rc{};
   rc.tbits = 16;
   const bool culled_bf = cull_bf && driver == DELTA_DRV_BF && precision == DELTA_F64;
-  if (culled_bf) rc.rel_slack = 1e-14;
-  if (culled_bf || driver == DELTA_DRV_BF_CERT || driver == DELTA_DRV_BF_CULLED || driver == DELTA_DRV_LEARNED)
-    st = detect_culled(ctx, culled_bf ? (int)DELTA_DRV_BF_CULLED : driver, m, pa, pb, n_pairs, cap, dev, host, pose, rc);
-  else
-    st = detect_rows(ctx, driver, precision, m, pa, pb, n_pairs, cap, dev, host, rc);
-  if (st != DELTA_OK) return st;
+  bool rows = !culled_bf && driver != DELTA_DRV_BF_CERT && driver != DELTA_DRV_BF_CULLED && driver != DELTA_DRV_LEARNED;
+  if (!rows) {
+    RawContacts cc = rc;
+    if (culled_bf) cc.rel_slack = 1e-14;
+    if ((st = detect_culled(ctx, culled_bf ? (int)DELTA_DRV_BF_CULLED : driver, m, pa, pb, n_pairs, cap, dev, host, pose,
+                            cc, culled_bf ? &rows : nullptr)) != DELTA_OK)
+      return st;
+    if (!rows) rc = cc;
+  }
+  if (rows && (st = detect_rows(ctx, driver, precision, m, pa, pb, n_pairs, cap, dev, host, rc)) != DELTA_OK) return st;
   const DevStats h = host->stats;
   if (counters) {
     counters[0] += (int64_t)h.tri_pairs;

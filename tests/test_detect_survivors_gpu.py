@@ -68,3 +68,48 @@ def test_a_long_survivor_list_is_kept_from_call_to_call(name):
         for f in FIELDS:
             assert np.array_equal(rows[f], want[f]), f
     assert runs[0][1] > least and [n for _, n in runs[1:]] == [least, least]
+
+
+@pytest.mark.parametrize("sizes,pairs", [
+    ([1, 1], [(0, 1)]),                                          # one slice
+    ([33, 600, 129, 2000], [(0, 1), (1, 0), (1, 2), (2, 3), (3, 1)]),  # slices with remainders, empty ones
+    ([1500, 1499], [(0, 1)]),
+    ([6000, 2], [(0, 1)]),                                       # second bodies too small to cut
+    ([60000, 2], [(0, 1)]),                                      # uneven: every triangle pair is solved
+    ([30] * 40 + [2500, 2500], [(k, k + 1) for k in range(39)] * 20 + [(40, 41)]),  # one large pair among small ones
+], ids=["one", "mixed", "pair", "flat", "flat_uneven", "uneven"])
+def test_bf_in_slices_equals_the_unsliced_culling(ctx, sizes, pairs):
+    """bf() culls slices of the second bodies, or solves every triangle pair where one large
+    body pair would hold up one block: the contacts of the culling with one block to a pair,
+    bit for bit."""
+    from delta_b200 import detection
+
+    m = bodies(sizes, seed=7, eps=2e-4 if max(sizes) < 100 else 2e-5)
+    got, _ = detect(ctx, detection.DRV_BF, m, pairs, detection.Contacts(1 << 17))
+    want, _ = detect(ctx, detection.DRV_BF_CULLED, m, pairs, detection.Contacts(1 << 17))
+    assert len(got) == len(want) and (len(want) > 0 or sum(sizes) < 10)
+    for f in FIELDS:
+        assert np.array_equal(got[f], want[f]), f
+
+
+def test_bf_on_two_large_bodies_uses_the_whole_chip(ctx):
+    """Two spheres of 5,120 triangles, one half inside the other: bf() took one block of the
+    culling 16 ms; in slices, or with every triangle pair solved, it takes less than half."""
+    import time
+
+    from delta_b200 import detection
+    from delta_b200.scenarios import sphere_mesh
+
+    V, F = sphere_mesh(5120, None, 0.5)
+    xyz = np.concatenate([V[F].reshape(-1, 3), (V + [0.3, 0.013, 0.007])[F].reshape(-1, 3)])
+    m = detection.Meshes(np.array([0, 5120, 10240]), *(xyz[:, k].copy() for k in range(3)), np.full(2, 1e-4),
+                         np.zeros(2, np.uint8))
+    least = {}
+    for driver in (detection.DRV_BF, detection.DRV_BF_CULLED):
+        contacts, times = detection.Contacts(4096), []
+        for _ in range(4):
+            t = time.perf_counter()
+            detect(ctx, driver, m, [(0, 1)], contacts)
+            times.append(time.perf_counter() - t)
+        least[driver] = min(times)
+    assert least[detection.DRV_BF] < 0.5 * least[detection.DRV_BF_CULLED], least
