@@ -1169,9 +1169,12 @@ static delta_status bad_argument(int bad) {
 // The culled drivers' contacts into rc, unordered: argument check, box culling into the
 // survivor list, the survivors' solver, all enqueued at once (after a failed check the
 // kernels that would read vertices return at once, and the solver finds no survivors; the
-// solver reads the survivors' number on the device); one read-back.  A buffer that was too small is grown
-// and the detection repeated.  With `rows` (bf()), *rows is set where the culling is not for
-// this list (cull_uneven) and nothing was detected.
+// solver reads the survivors' number on the device); one read-back.  A buffer that was too
+// small is grown and the detection repeated.  With `rows` (bf()), *rows is set where the
+// culling is not for this list (cull_uneven, or more survivors than kMaxSurvivors or than
+// there is memory for) and nothing was detected: every triangle pair can be solved without a
+// list.
+constexpr int64_t kMaxSurvivors = 1 << 26;  // 512 MB, at least 15 ms of the solver
 static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes &m, const int32_t *pa,
                                   const int32_t *pb, int64_t n_pairs, int64_t cap, DetectSmall *dev,
                                   DetectSmall *host, const Pose *pose, RawContacts &rc, bool *rows) {
@@ -1198,9 +1201,15 @@ static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes
   int64_t sv_cap = std::max<int64_t>(std::max<int64_t>(8 * cap, 1 << 16),
                                      (int64_t)(ctx->scratch[9].bytes / sizeof(uint64_t)));
   for (;;) {
+    if (rows) sv_cap = std::min(sv_cap, kMaxSurvivors);
     if ((st = raw_contacts(ctx, cap, rc)) != DELTA_OK) return st;
     void *svb = nullptr;
-    if ((st = ctx_scratch(ctx, 9, sizeof(uint64_t) * (size_t)sv_cap, &svb)) != DELTA_OK) return st;
+    if ((st = ctx_scratch(ctx, 9, sizeof(uint64_t) * (size_t)sv_cap, &svb)) != DELTA_OK) {
+      if (!rows || st != DELTA_ERR_NOMEM) return st;
+      cudaGetLastError();
+      *rows = true;
+      return DELTA_OK;
+    }
     rc.sv = (uint64_t *)svb;
     rc.sv_cap = sv_cap;
     if ((e = cudaMemsetAsync(dev, 0, sizeof(DetectSmall), s)) != cudaSuccess) return cuda_error(e, "detect memset");
@@ -1227,6 +1236,7 @@ static delta_status detect_culled(delta_ctx *ctx, int driver, const delta_meshes
     if (rows && (*rows = cull_uneven(host->work, n_pairs))) return DELTA_OK;
     host->stats.evaluated = host->sv_count;
     const int64_t nsv = (int64_t)host->sv_count, nc = (int64_t)host->count;
+    if (rows && (*rows = nsv > kMaxSurvivors)) return DELTA_OK;
     if (nsv > sv_cap) sv_cap = nsv + nsv / 4;
     else if (nc > cap) cap = nc + nc / 4;
     else return DELTA_OK;

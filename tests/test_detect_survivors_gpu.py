@@ -113,3 +113,29 @@ def test_bf_on_two_large_bodies_uses_the_whole_chip(ctx):
             times.append(time.perf_counter() - t)
         least[driver] = min(times)
     assert least[detection.DRV_BF] < 0.5 * least[detection.DRV_BF_CULLED], least
+
+
+def test_bf_bounds_its_survivor_list():
+    """bf() needs no memory for the triangle pairs that it solves one by one, so the list of its
+    culling is bounded: four pairs with 77 million survivors (0.6 GB) are solved without one.
+    The contacts are those of the driver that lists them all."""
+    import torch
+
+    from delta_b200 import detection
+    from delta_b200.narrowphase import Context
+
+    m = bodies([4400] * 5, seed=11, eps=1e-7)
+    pairs = [(k, k + 1) for k in range(4)]
+    rows = {}
+    for driver in (detection.DRV_BF, detection.DRV_BF_CULLED):
+        ctx, contacts = Context(0), detection.Contacts(1 << 17)
+        free = torch.cuda.mem_get_info()[0]
+        rows[driver], _ = detect(ctx, driver, m, pairs, contacts)
+        used = free - torch.cuda.mem_get_info()[0]
+        ctx.close()
+        if driver == detection.DRV_BF:
+            assert used < 200 << 20, used
+    got, want = rows.values()
+    assert len(got) == len(want) > 0
+    for f in FIELDS:
+        assert np.array_equal(got[f], want[f]), f
