@@ -1601,13 +1601,19 @@ __global__ void k_unpack_selected(const uint64_t *__restrict__ sel, const int64_
 // index), so that a search step is one load where the grid kernels follow three pointers;
 // every atomic's return value is the rank of its element, so that placing needs no second
 // one; and the pairs are ordered by a counting sort over their first body and a rank within
-// its run (a moving body's few neighbours; an obstacle's run may be long).
+// its run (a moving body's few neighbours; an obstacle's run may be long, see kSkinLongRun).
 constexpr int kSkinMaxCtas = 16, kSkinThreads = 1024;
 constexpr int kSkinRounds = 4;  // entries per thread
 constexpr int64_t kSkinClusterCap = (int64_t)8 * kSkinThreads * kSkinRounds;
 // Scenes of more bodies keep the conditional node: a build by 16 SMs takes too long there.
 constexpr int32_t kSkinClusterBodies = 1 << 16;
 constexpr int kSkinBoxes = 128;  // obstacle boxes staged at a time
+// A run of the build's pairs (one first body) longer than this is ordered by a CTA with a
+// bitmap of the second bodies, not by counting, whose work is the run's length squared: with
+// the floor as body 0 and 16,000 bodies on it, a step with a rebuild took 705 us (119 with the
+// floor as the last body), now 137.
+constexpr uint32_t kSkinLongRun = 512;
+constexpr int kSkinWords = kSkinClusterBodies / 32;
 
 struct SkinRecord {
   double x, y, z, reach;  // centre, radius + eps
@@ -1656,6 +1662,9 @@ struct SkinStepSmem {
   uint32_t part[kSkinMaxCtas];  // the build's scans: each CTA's total
   uint32_t wsum[32];
   double box[kSkinBoxes][7];    // obstacle boxes and eps
+  int runs;                     // long runs whose first pair this CTA met, and their first bodies
+  int run[kSkinClusterCap / kSkinLongRun];
+  uint32_t bits[kSkinWords], below[kSkinWords];  // second bodies of a long run; those in lower words
 };
 
 // The cluster's barrier (release and acquire: the CTAs' global writes before it are visible
@@ -1719,6 +1728,46 @@ __device__ __forceinline__ void push_ranked(int32_t a, int32_t b, int sh, const 
   }
 }
 
+// The pairs of one first body, from k.sel to k.keys in order, by the whole CTA: a pair's rank
+// is the number of set bits below its second body's.
+__device__ __forceinline__ void cluster_long_run(SkinStepSmem &sm, const SkinList &k, const SkinBuild &bd, int body,
+                                                 int32_t n, int sh) {
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const uint32_t lo = __ldcg(bd.astart + body), hi = __ldcg(bd.astart + body + 1);
+  const uint64_t low = (1ull << sh) - 1ull;
+  const int words = (n + 31) / 32, each = (words + kSkinThreads - 1) / kSkinThreads;
+  for (int i = t; i < words; i += kSkinThreads) sm.bits[i] = 0u;
+  __syncthreads();
+  for (uint32_t q = lo + t; q < hi; q += kSkinThreads) {
+    const uint32_t b = (uint32_t)(__ldcg(k.sel + q) & low);
+    atomicOr(&sm.bits[b >> 5], 1u << (b & 31));
+  }
+  __syncthreads();
+  uint32_t own = 0;
+  for (int i = t * each; i < (t + 1) * each && i < words; ++i) own += __popc(sm.bits[i]);
+  uint32_t incl = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) sm.wsum[w] = incl;
+  __syncthreads();
+  uint32_t at = incl - own;
+  for (int c = 0; c < w; ++c) at += sm.wsum[c];
+  for (int i = t * each; i < (t + 1) * each && i < words; ++i) {
+    sm.below[i] = at;
+    at += __popc(sm.bits[i]);
+  }
+  __syncthreads();
+  for (uint32_t q = lo + t; q < hi; q += kSkinThreads) {
+    const uint64_t key = __ldcg(k.sel + q);
+    const uint32_t b = (uint32_t)(key & low);
+    k.keys[lo + sm.below[b >> 5] + __popc(sm.bits[b >> 5] & ((1u << (b & 31)) - 1u))] = key;
+  }
+  __syncthreads();  // the bitmap and the sums are used again
+}
+
 // The list rebuilt at the current positions: the pairs within reach + skin of skin_build's
 // search (k_grid_pairs, k_obstacle_pairs; the reaches are added in another order, which the
 // test's margins cover), in key order.
@@ -1731,6 +1780,7 @@ __device__ __forceinline__ void cluster_skin_build(SkinStepSmem &sm, const delta
   const int32_t n = s.n_bodies;
   // 1. cells, buckets and ranks
   if (t == 0) *k.raw_count = 0ull;
+  if (threadIdx.x == 0) sm.runs = 0;
   for (int64_t i = t; i < n; i += T) {
     if (s.obstacle[i]) continue;
     int64_t c[3];
@@ -1836,12 +1886,18 @@ __device__ __forceinline__ void cluster_skin_build(SkinStepSmem &sm, const delta
     }
     const uint64_t key = __ldcg(k.sel + i);
     const uint32_t lo = __ldcg(bd.astart + (key >> sh)), hi = __ldcg(bd.astart + (key >> sh) + 1);
+    if (hi - lo > kSkinLongRun) {
+      if (i == lo) sm.run[atomicAdd(&sm.runs, 1)] = (int)(key >> sh);
+      continue;
+    }
     uint32_t r = lo;
 #pragma unroll 8
     for (uint32_t q = lo; q < hi; ++q) r += __ldcg(k.sel + q) < key ? 1u : 0u;
     k.keys[r] = key;
   }
   for (int64_t i = t; i < 3 * (int64_t)n; i += T) k.anchor[i] = s.pos[i];
+  __syncthreads();
+  for (int x = 0; x < sm.runs; ++x) cluster_long_run(sm, k, bd, sm.run[x], n, sh);
   if (t == 0) {
     *k.need = 0;
     *k.rebuilds += 1ull;

@@ -1,0 +1,108 @@
+"""The graph step's skin list where its cost depends on the scene: the order of the bodies, the
+number of obstacles, the number of bodies. Results are compared with delta_sim_step bit for
+bit; times only with those of a like scene, by ratios far from what was measured."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BODY_STATE = ("pos", "vel", "ang", "ref_ang", "rot")
+STATE = BODY_STATE + ("x", "y", "z")
+DRV_CERT = 8
+
+
+def permuted(scene, order):
+    """The scene with its bodies in another order."""
+    n, off = scene["n_bodies"], scene["tri_offset"]
+    count = np.diff(off)[order]
+    tri = np.concatenate([np.arange(off[b], off[b + 1]) for b in order])
+    vertex = (3 * tri[:, None] + np.arange(3)).reshape(-1)
+    out = {"n_bodies": n, "tri_offset": np.concatenate([[0], np.cumsum(count)]).astype(np.int64),
+           "tri_body": np.repeat(np.arange(n, dtype=np.int32), count)}
+    for k, a in scene.items():
+        if k in ("x", "y", "z", "rx", "ry", "rz"):
+            out[k] = a[vertex].copy()
+        elif k not in out:
+            out[k] = np.asarray(a).reshape(n, -1)[order].reshape(-1).copy()
+    return out
+
+
+def layer(n, floor_first=False, spacing=0.03, height=0.0104):
+    """n particles of 20 triangles in one layer, the skin's reach above a floor of two."""
+    from delta_b200.scenarios import particle_cloud_scene
+
+    side = int(np.ceil(np.sqrt(n)))
+    k, h = np.arange(n), 0.6 * side * spacing + 1.0
+    centres = np.stack([(k % side - side / 2) * spacing, np.full(n, height), (k // side - side / 2) * spacing], 1)
+    floor = (np.array([[-h, 0, -h], [h, 0, -h], [h, 0, h], [-h, 0, h]], float), np.array([[0, 2, 1], [0, 3, 2]]))
+    scene = particle_cloud_scene(centres, np.full(n, 0.01), np.full(n, 20), [floor], seed=3, perturb=(1.0, 1.0))
+    return permuted(scene, np.concatenate([[n], np.arange(n)])) if floor_first else scene
+
+
+def moving(scene, velocity):
+    """The scene with its particles at `velocity` (3,) or (n, 3)."""
+    v = np.zeros((scene["n_bodies"], 3))
+    v[scene["obstacle"] == 0] = velocity
+    scene["vel"] = v.reshape(-1).copy()
+    return scene
+
+
+def same_run(ctx, scene, steps, dt=1e-5, driver=DRV_CERT):
+    """`steps` graph steps in one call equal single steps; returns (skin statistics, contacts)."""
+    from delta_b200.engine import Simulation, StepParams
+
+    prm = StepParams.make(dt=dt, gravity=(0.0, 0.0, 0.0))
+    runs = []
+    for graph in (False, True):
+        sim = Simulation(ctx, scene, driver)
+        cps = sim.step(steps, prm, graph=graph)
+        runs.append((cps, sim.state(), sim.counters()))
+        skin = sim.skin_stats()
+        sim.close()
+    (c0, s0, n0), (c1, s1, n1) = runs
+    assert np.array_equal(c0, c1)
+    for k in STATE:
+        assert np.array_equal(s0[k], s1[k]), k
+    for k in ("steps", "body_pairs", "triangle_pairs", "solved"):
+        assert n0[k] == n1[k], k
+    return skin, int(c1.sum())
+
+
+def rebuilding_step(ctx, scene, steps=48):
+    """Seconds a step when every step rebuilds the list (the bodies cross half the skin)."""
+    from delta_b200.engine import Simulation, StepParams
+
+    prm = StepParams.make(dt=1e-5, gravity=(0.0, 0.0, 0.0))
+    sim = Simulation(ctx, scene, DRV_CERT)
+    sim.step(1, prm, graph=True)
+    skin = sim.skin_stats()["skin"]
+    sim.close()
+    sim = Simulation(ctx, moving(dict(scene), [0.75 * skin / 1e-5, 0.0, 0.0]), DRV_CERT)
+    start = {k: sim.dev.t[k].clone() for k in BODY_STATE}
+    best = np.inf
+    for _ in range(4):
+        for k, v in start.items():
+            sim.dev.t[k].copy_(v)
+        t = time.perf_counter()
+        sim.step(steps, prm, graph=True)
+        best = min(best, time.perf_counter() - t)
+    assert sim.skin_stats()["rebuilds"] >= 4 * (steps - 1)
+    sim.close()
+    return best / steps
+
+
+@pytest.mark.parametrize("n", [513, 700, 5000])
+def test_a_floor_as_the_first_body_is_ordered(ctx, n):
+    """The floor's run of pairs (one first body) is longer than 512, and ordered by the bitmap."""
+    rng = np.random.default_rng(n)
+    scene = moving(layer(n, floor_first=True, height=0.0084), rng.uniform(-40.0, 40.0, (n, 3)) * (1.0, 0.05, 1.0))
+    skin, contacts = same_run(ctx, scene, 12)
+    assert skin["rebuilds"] >= 3 and contacts > 0, (skin, contacts)
+
+
+def test_a_rebuild_costs_the_same_whichever_body_the_floor_is(ctx):
+    """Counting ranked a run by its length squared: with the floor as the first body, 12,000
+    particles on it, a step with a rebuild took 4 times that with the floor as the last."""
+    assert rebuilding_step(ctx, layer(12000, floor_first=True)) < 2.0 * rebuilding_step(ctx, layer(12000))
