@@ -1608,6 +1608,15 @@ constexpr int64_t kSkinClusterCap = (int64_t)8 * kSkinThreads * kSkinRounds;
 // Scenes of more bodies keep the conditional node: a build by 16 SMs takes too long there.
 constexpr int32_t kSkinClusterBodies = 1 << 16;
 constexpr int kSkinBoxes = 128;  // obstacle boxes staged at a time
+// Up to this many obstacles, a build tests every body against every box, a thread a body; with
+// more (kManyBoxes) it tells most of them apart in FP32 and shares them out.  Microseconds of a
+// step with a rebuild, first way / second, at 1,000, 4,000 and 16,000 bodies:
+//   1 box      69 / 72   87 / 92  139 / 147
+//   24 boxes   72 / 74   94 / 93  144 / 148
+//   32         68 / 61   97 / 92  145 / 150
+//   128        96 / 62  112 / 83  173 / 166
+//   1,000     359 / 84  373 / 132 410 / 300
+constexpr int32_t kSkinFewBoxes = 24;
 // A run of the build's pairs (one first body) longer than this is ordered by a CTA with a
 // bitmap of the second bodies, not by counting, whose work is the run's length squared: with
 // the floor as body 0 and 16,000 bodies on it, a step with a rebuild took 705 us (119 with the
@@ -1662,6 +1671,7 @@ struct SkinStepSmem {
   uint32_t part[kSkinMaxCtas];  // the build's scans: each CTA's total
   uint32_t wsum[32];
   double box[kSkinBoxes][7];    // obstacle boxes and eps
+  alignas(16) float far_box[kSkinBoxes][8];  // their lo at 0, hi at 4, rounded outwards
   int runs;                     // long runs whose first pair this CTA met, and their first bodies
   int run[kSkinClusterCap / kSkinLongRun];
   uint32_t bits[kSkinWords], below[kSkinWords];  // second bodies of a long run; those in lower words
@@ -1771,6 +1781,7 @@ __device__ __forceinline__ void cluster_long_run(SkinStepSmem &sm, const SkinLis
 // The list rebuilt at the current positions: the pairs within reach + skin of skin_build's
 // search (k_grid_pairs, k_obstacle_pairs; the reaches are added in another order, which the
 // test's margins cover), in key order.
+template <bool kManyBoxes>
 __device__ __forceinline__ void cluster_skin_build(SkinStepSmem &sm, const delta_scene &s, const Grid &g,
                                                    const SkinBuild &bd, const SkinList &k, int sh,
                                                    const int32_t *obst, const double *box, int32_t n_obst,
@@ -1804,9 +1815,12 @@ __device__ __forceinline__ void cluster_skin_build(SkinStepSmem &sm, const delta
   // order; the obstacle boxes against every body
   for (int64_t i = t; i < bd.nb + 1; i += T) bd.bcount[i] = 0u;
   const int64_t moving = __ldcg(bd.bstart + bd.nb);
-  auto within = [&](double d2, double reach) {
+  auto widened = [&](double reach) {
     reach = reach * (1.0 + 1e-9) + 1e-12;
-    reach = (reach + skin) * (1.0 + 1e-9) + 1e-12;
+    return (reach + skin) * (1.0 + 1e-9) + 1e-12;
+  };
+  auto within = [&](double d2, double reach) {
+    reach = widened(reach);
     return d2 <= reach * reach;
   };
   auto load_rec = [&](int64_t q) {
@@ -1852,18 +1866,53 @@ __device__ __forceinline__ void cluster_skin_build(SkinStepSmem &sm, const delta
     __syncthreads();
     for (int i = threadIdx.x; i < 7 * no; i += kSkinThreads)
       sm.box[i / 7][i % 7] = i % 7 < 6 ? box[6 * (int64_t)(o0 + i / 7) + i % 7] : s.eps[obst[o0 + i / 7]];
+    if constexpr (kManyBoxes)
+      for (int i = threadIdx.x; i < 6 * no; i += kSkinThreads) {
+        const int o = i / 6, d = i % 6;
+        const double x = box[6 * (int64_t)(o0 + o) + d];
+        sm.far_box[o][d < 3 ? d : d + 1] = d < 3 ? __double2float_rd(x) : __double2float_ru(x);
+      }
     __syncthreads();
-    for (int64_t e = t; e < moving; e += T) {
-      const SkinRecord me = load_rec(e);
+    auto search = [&](const SkinRecord &me, int64_t e, int32_t o) {
       const double c[3] = {me.x, me.y, me.z};
-      for (int32_t o = 0; o < no; ++o) {
-        double d2 = 0.0;
+      double d2 = 0.0;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const double gap = fmax(sm.box[o][d] - c[d], c[d] - sm.box[o][3 + d]);
-          if (gap > 0.0) d2 += gap * gap;
+      for (int d = 0; d < 3; ++d) {
+        const double gap = fmax(sm.box[o][d] - c[d], c[d] - sm.box[o][3 + d]);
+        if (gap > 0.0) d2 += gap * gap;
+      }
+      if (within(d2, me.reach + sm.box[o][6])) push_ranked(obst[o0 + o], (int32_t)load_cell(e).body, sh, k, bd);
+    };
+    if constexpr (!kManyBoxes) {
+      for (int64_t e = t; e < moving; e += T) {
+        const SkinRecord me = load_rec(e);
+        for (int32_t o = 0; o < no; ++o) search(me, e, o);
+      }
+    } else {
+      // most boxes are told apart in FP32, box and body's reach rounded outwards, and they are
+      // shared out between `groups` threads a body where there are fewer bodies than threads
+      const uint32_t m = (uint32_t)moving, groups = m > 0 && m < T ? (uint32_t)T / m : 1u;
+      for (uint32_t w = (uint32_t)t; w < groups * m; w += (uint32_t)T) {
+        const uint32_t g0 = groups > 1 ? w / m : 0u, e = w - g0 * m;
+        const SkinRecord me = load_rec(e);
+        const double c[3] = {me.x, me.y, me.z};
+        double eps = NAN;  // of the boxes that lo and hi are for
+        float lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
+        for (int32_t o = (int32_t)g0; o < no; o += (int32_t)groups) {
+          if (sm.box[o][6] != eps) {
+            eps = sm.box[o][6];
+            const double far = widened(me.reach + eps);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              lo[d] = __double2float_rd(c[d] - far);
+              hi[d] = __double2float_ru(c[d] + far);
+            }
+          }
+          const float4 bl = *reinterpret_cast<const float4 *>(&sm.far_box[o][0]);
+          const float4 bh = *reinterpret_cast<const float4 *>(&sm.far_box[o][4]);
+          if (bl.x > hi[0] || bh.x < lo[0] || bl.y > hi[1] || bh.y < lo[1] || bl.z > hi[2] || bh.z < lo[2]) continue;
+          search(me, e, o);
         }
-        if (within(d2, me.reach + sm.box[o][6])) push_ranked(obst[o0 + o], (int32_t)load_cell(e).body, sh, k, bd);
       }
     }
   }
@@ -1905,6 +1954,7 @@ __device__ __forceinline__ void cluster_skin_build(SkinStepSmem &sm, const delta
   skin_sync();
 }
 
+template <bool kManyBoxes>
 __global__ void __launch_bounds__(kSkinThreads, 1)
     k_skin_step(delta_scene s, Grid g, SkinBuild bd, SkinList k, SkinTouch touch, const int32_t *obst, int32_t n_obst,
                 double skin, double limit2, int32_t *pa, int32_t *pb, int64_t pair_cap,
@@ -1972,7 +2022,7 @@ __global__ void __launch_bounds__(kSkinThreads, 1)
     int need = 0;
     for (int c = 0; c < ctas; ++c) need |= sm.need[c];
     if (!need) break;
-    cluster_skin_build(sm, s, g, bd, k, touch.sh, obst, touch.box, n_obst, skin, ovf);
+    cluster_skin_build<kManyBoxes>(sm, s, g, bd, k, touch.sh, obst, touch.box, n_obst, skin, ovf);
     rebuilt = true;  // (the build ends with a barrier: sum and need are free to be sent again)
   }
   int before = 0, found = 0;
@@ -2004,8 +2054,9 @@ static bool skin_cluster(int32_t n, int64_t cap) { return cap > 0 && cap <= kSki
 
 // CTAs of k_skin_step's cluster: 16 (beyond the portable 8, so asked for) where they can be
 // resident together.
+template <bool kManyBoxes>
 static cudaError_t skin_cluster_size(int *ctas) {
-  cudaError_t e = cudaFuncSetAttribute(k_skin_step, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaError_t e = cudaFuncSetAttribute(k_skin_step<kManyBoxes>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(kSkinMaxCtas);
@@ -2017,7 +2068,7 @@ static cudaError_t skin_cluster_size(int *ctas) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaOccupancyMaxActiveClusters(&clusters, k_skin_step, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&clusters, k_skin_step<kManyBoxes>, &cfg) != cudaSuccess) {
     cudaGetLastError();
     clusters = 0;
   }
@@ -2410,7 +2461,8 @@ static delta_status graph_alloc(delta_sim *s, int64_t pair_cap, int64_t contact_
     if (cluster) {
       const SkinBuild bd = carve_skin_build(g.skin.anchor + 3 * (size_t)n, n, cap);
       if ((e = cudaMemset(bd.bcount, 0, 4 * ((size_t)bd.nb + n + 2))) != cudaSuccess ||
-          (e = skin_cluster_size(&g.skin_ctas)) != cudaSuccess)
+          (e = s->plan.n_obst > kSkinFewBoxes ? skin_cluster_size<true>(&g.skin_ctas)
+                                              : skin_cluster_size<false>(&g.skin_ctas)) != cudaSuccess)
         return cuda_error(e, "skin build state");
     }
     g.skin.need = &g.state->need;
@@ -2429,8 +2481,9 @@ static delta_status graph_skin_cluster(delta_sim *s, int &k) {
   delta_sim::Graph &g = s->g;
   const BroadphasePlan &plan = s->plan;
   const double limit = 0.5 * plan.skin * (1.0 - 1e-9);
+  auto kernel = plan.n_obst > kSkinFewBoxes ? k_skin_step<true> : k_skin_step<false>;
   const cudaError_t e = launch_dep_cluster(
-      k_skin_step, (unsigned)g.skin_ctas, kSkinThreads, g.stream, s->scene, plan.gs,
+      kernel, (unsigned)g.skin_ctas, kSkinThreads, g.stream, s->scene, plan.gs,
       carve_skin_build(g.skin.anchor + 3 * (size_t)s->scene.n_bodies, s->scene.n_bodies, g.skin.cap), g.skin,
       skin_touch(s->scene, plan), plan.d_obst, plan.n_obst, plan.skin, limit * limit, g.pa, g.pb, g.pair_cap,
       broadphase_fixed_count(g.bp, s->scene.n_bodies), g.d_ovf, g.d_pend);

@@ -41,6 +41,23 @@ def layer(n, floor_first=False, spacing=0.03, height=0.0104):
     return permuted(scene, np.concatenate([[n], np.arange(n)])) if floor_first else scene
 
 
+def shelves(n, m, seed=0):
+    """n particles of 20 triangles in a cube, and m small plates, most of them just under one."""
+    from delta_b200.scenarios import particle_cloud_scene
+
+    rng = np.random.default_rng(seed)
+    side = int(np.ceil(n ** (1 / 3)))
+    k = np.arange(n)
+    centres = 0.03 * np.stack([k % side, k // (side * side), k // side % side], 1).astype(float)
+    under = centres[rng.integers(0, n, m)] - [0.0, 0.0086, 0.0]
+    under[rng.random(m) < 0.3] += 5.0
+    plate = np.array([[-1, 0, -1], [1, 0, -1], [1, 0, 1], [-1, 0, 1]], float)
+    plates = [(u + w * plate, np.array([[0, 2, 1], [0, 3, 2]])) for u, w in zip(under, rng.uniform(0.002, 0.05, m))]
+    scene = particle_cloud_scene(centres, np.full(n, 0.01), np.full(n, 20), plates, seed=3, perturb=(1.0, 1.0))
+    scene["eps"] = np.where(scene["obstacle"] != 0, rng.choice([1e-4, 2e-4, 3e-4], n + m), 1e-4)
+    return scene
+
+
 def moving(scene, velocity):
     """The scene with its particles at `velocity` (3,) or (n, 3)."""
     v = np.zeros((scene["n_bodies"], 3))
@@ -106,3 +123,28 @@ def test_a_rebuild_costs_the_same_whichever_body_the_floor_is(ctx):
     """Counting ranked a run by its length squared: with the floor as the first body, 12,000
     particles on it, a step with a rebuild took 4 times that with the floor as the last."""
     assert rebuilding_step(ctx, layer(12000, floor_first=True)) < 2.0 * rebuilding_step(ctx, layer(12000))
+
+
+@pytest.mark.parametrize("n,m", [(3, 25), (700, 24), (700, 25), (2000, 128), (5000, 129), (9000, 300)])
+def test_many_obstacles_are_all_searched(ctx, n, m):
+    """Obstacle boxes shared out between threads (fewer particles than threads: 5, 8 and 3
+    groups) or not (9,000 particles), in stages of 128, with several margins among them."""
+    rng = np.random.default_rng(n)
+    scene = moving(shelves(n, m, seed=m), rng.uniform(-30.0, 30.0, (n, 3)))
+    skin, contacts = same_run(ctx, scene, 12)
+    assert skin["rebuilds"] >= 3 and contacts > 0, (skin, contacts)
+
+
+def test_a_rebuild_with_many_obstacles_costs_little_more(ctx):
+    """Every box was tested against every particle by one thread a particle: a step with a
+    rebuild, 1,000 particles, took 5 times as long with 1,000 far obstacles as with none."""
+    from delta_b200.scenarios import particle_cloud_scene
+
+    def scene(m):
+        k = np.arange(1000)
+        centres = 0.03 * np.stack([k % 10, k // 100, k // 10 % 10], 1).astype(float)
+        quad = np.array([[-9, 0, -9], [9, 0, -9], [9, 0, 9], [-9, 0, 9]], float)
+        floors = [(quad - [0, 0.05 + 0.01 * i, 0], np.array([[0, 2, 1], [0, 3, 2]])) for i in range(m)]
+        return particle_cloud_scene(centres, np.full(1000, 0.01), np.full(1000, 20), floors, seed=3)
+
+    assert rebuilding_step(ctx, scene(1000)) < 2.5 * rebuilding_step(ctx, scene(1))
