@@ -1605,8 +1605,19 @@ __global__ void k_unpack_selected(const uint64_t *__restrict__ sel, const int64_
 constexpr int kSkinMaxCtas = 16, kSkinThreads = 1024;
 constexpr int kSkinRounds = 4;  // entries per thread
 constexpr int64_t kSkinClusterCap = (int64_t)8 * kSkinThreads * kSkinRounds;
-// Scenes of more bodies keep the conditional node: a build by 16 SMs takes too long there.
-constexpr int32_t kSkinClusterBodies = 1 << 16;
+// Scenes of more bodies, or of more bodies times obstacles, keep the conditional node: a build
+// by 16 SMs takes longer than one by the whole chip, a step without a build is shorter.  The
+// lines lie about where one step in ten builds costs the same.  Microseconds a step, node /
+// cluster, without and with a build:
+//   4,000 bodies     34 / 27    86 /  87
+//   8,000            35 / 28    89 / 104
+//   16,000           37 / 31    92 / 139
+//   20,000           37 / 32    81 / 143
+//   32,000           41 / 37    91 / 209
+//   8,000 bodies and 1,000 obstacles   36 / 31   121 / 191
+//   16,000 and 1,000                   39 / 35   154 / 300
+constexpr int32_t kSkinClusterBodies = 1 << 14;
+constexpr int64_t kSkinClusterTests = 1 << 23;
 constexpr int kSkinBoxes = 128;  // obstacle boxes staged at a time
 // Up to this many obstacles, a build tests every body against every box, a thread a body; with
 // more (kManyBoxes) it tells most of them apart in FP32 and shares them out.  Microseconds of a
@@ -2049,8 +2060,11 @@ __global__ void __launch_bounds__(kSkinThreads, 1)
   }
 }
 
-// Whether a scene's skin list is handled by one cluster.
-static bool skin_cluster(int32_t n, int64_t cap) { return cap > 0 && cap <= kSkinClusterCap && n <= kSkinClusterBodies; }
+// Whether a scene's skin list, of capacity cap, is handled by one cluster.
+static bool skin_cluster(const delta_scene &s, const BroadphasePlan &plan, int64_t cap) {
+  return cap > 0 && cap <= kSkinClusterCap && s.n_bodies <= kSkinClusterBodies &&
+         (int64_t)plan.n_moving * plan.n_obst <= kSkinClusterTests;
+}
 
 // CTAs of k_skin_step's cluster: 16 (beyond the portable 8, so asked for) where they can be
 // resident together.
@@ -2454,7 +2468,7 @@ static delta_status graph_alloc(delta_sim *s, int64_t pair_cap, int64_t contact_
       if ((e = cudaMalloc(&g.temp, tb)) != cudaSuccess) return cuda_error(e, "skin temp");
       g.temp_bytes = tb;
     }
-    const bool cluster = skin_cluster(n, cap);
+    const bool cluster = skin_cluster(s->scene, s->plan, cap);
     if ((e = cudaMalloc(&g.sk, skin_bytes(n, cap) + (cluster ? skin_build_bytes(n, cap) : 0))) != cudaSuccess)
       return cuda_error(e, "skin list");
     g.skin = carve_skin(g.sk, n, cap);
@@ -2559,7 +2573,7 @@ static delta_status graph_enqueue_step(delta_sim *s, const delta_step_params &p,
   cudaError_t le = launch_dep(true, k_bodies, blocks_for(s->scene.n_bodies, 128), 128, 0, st, s->scene, p, s->F, s->T,
                               s->has, g.d_ovf, g.d_snap, s->epoch);
   if (le != cudaSuccess) return cuda_error(le, "body update");
-  if (skin_cluster(s->scene.n_bodies, g.skin.cap)) {
+  if (skin_cluster(s->scene, s->plan, g.skin.cap)) {
     if ((ds = graph_skin_cluster(s, k)) != DELTA_OK) return ds;
   } else if (g.skin.cap > 0) {
     if ((ds = graph_skin_broadphase(s, k)) != DELTA_OK) return ds;

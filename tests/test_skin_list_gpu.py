@@ -148,3 +148,56 @@ def test_a_rebuild_with_many_obstacles_costs_little_more(ctx):
         return particle_cloud_scene(centres, np.full(1000, 0.01), np.full(1000, 20), floors, seed=3)
 
     assert rebuilding_step(ctx, scene(1000)) < 2.5 * rebuilding_step(ctx, scene(1))
+
+
+def kernels_of_a_step(ctx, scene):
+    """Kernels in a replayed step without a rebuild."""
+    from delta_b200 import lib
+    from delta_b200.engine import Simulation, StepParams
+
+    prm = StepParams.make(dt=1e-9, gravity=(0.0, 0.0, 0.0))
+    sim = Simulation(ctx, scene, DRV_CERT)
+    sim.step(2, prm, graph=True)
+    counts = []
+    for steps in (8, 24):
+        before = lib().delta_launch_count(ctx.handle)
+        sim.step(steps, prm, graph=True)
+        counts.append(lib().delta_launch_count(ctx.handle) - before)
+    sim.close()
+    return (counts[1] - counts[0]) // 16
+
+
+def test_the_route_changes_with_the_bodies_and_the_obstacles(ctx):
+    """Up to 16,384 bodies and 2^23 bodies times obstacles one cluster keeps the list; beyond,
+    the conditional node, whose check and filter are more kernels a step."""
+    small = kernels_of_a_step(ctx, layer(16383))  # and the floor
+    assert kernels_of_a_step(ctx, layer(16384)) > small
+    assert kernels_of_a_step(ctx, shelves(8192, 1024)) == small
+    assert kernels_of_a_step(ctx, shelves(8192, 1025)) > small
+
+
+@pytest.mark.parametrize("kind", ["sparse", "long", "overflow"])
+def test_the_conditional_node_equals_stepping(ctx, kind):
+    """The skin list's other route, over rebuilds caused by motion inside graphs of eight steps
+    and of one, with counters: more than 16,384 bodies and a short list (sorted and compacted
+    by one CTA); a list above 32,768 keys (sorted and selected by the whole chip); a lattice
+    squeezed until its list outgrows the capacity it got from the first, empty search."""
+    from delta_b200.scenarios import particle_cloud_scene
+
+    rng = np.random.default_rng(31)
+    side, spacing, steps = {"sparse": (26, 0.05, 27), "long": (21, 0.0206, 27), "overflow": (26, 0.027, 115)}[kind]
+    g = (np.arange(side) - (side - 1) / 2) * spacing
+    cen = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+    n = len(cen)
+    if kind == "sparse":
+        cen[1:400:2] = cen[0:400:2] + [0.018, 0.0, 0.0]  # 200 pairs that touch
+    scene = particle_cloud_scene(cen, np.full(n, 0.0095 if kind == "overflow" else 0.01), np.full(n, 20), [], seed=9)
+    scene = moving(scene, -300.0 * cen if kind == "overflow" else rng.uniform(-20.0, 20.0, (n, 3)))
+    skin, contacts = same_run(ctx, scene, steps)
+    assert contacts > 0
+    if kind == "sparse":
+        assert n > 16384 and skin["rebuilds"] >= 3 and skin["capacity"] <= 8192, skin
+    elif kind == "long":
+        assert skin["rebuilds"] >= 3 and skin["capacity"] > 32768, skin
+    else:
+        assert skin["capacity"] > 8192, skin  # grown past the first list's
