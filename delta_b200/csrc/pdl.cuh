@@ -8,8 +8,13 @@
 // the kernel reads or writes is touched before then; griddepcontrol.launch_dependents then
 // lets the next kernel's launch begin.  What overlaps is the launch and block scheduling of
 // a kernel with the end of the one before it.  Launched without the attribute (the stepped
-// path), dep_sync() returns at once.  No kernel launched this way waits on another CTA, so
-// CTAs of a dependent kernel that are resident early cannot hold up the kernel before it.
+// path), dep_sync() returns at once.
+//
+// CTAs of a dependent kernel that are resident early cannot hold up the kernel before it: they
+// become resident only when all of that kernel's CTAs have issued launch_dependents, so each
+// of them runs already.  A kernel of launch_dep waits on no other CTA of its own either; one
+// whose CTAs do is one cluster (launch_dep_cluster), which the hardware starts as a whole, and
+// its dependents start only when all of its CTAs have issued launch_dependents.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -44,7 +49,8 @@ inline cudaError_t launch_dep(bool dep, void (*kernel)(KArgs...), dim3 grid, dim
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// kernel as one cluster of `ctas` CTAs, a programmatic dependent launch.
+// kernel as one cluster of `ctas` CTAs, a programmatic dependent launch; its CTAs may wait on
+// one another.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dep_cluster(void (*kernel)(KArgs...), unsigned ctas, unsigned block, cudaStream_t st,
                                       Args &&...args) {
