@@ -9,7 +9,9 @@
 //        d_true >= |r| + min_{corners c of the parameter domain} grad|r| . (c - (s,t))
 //    holds whatever (s,t) is, so inexact FP32 parameters only loosen the bound.  The
 //    band eps = 64 u32 L (L = extent of the pair's bounding box) covers the rounding of
-//    the inputs and of the FP32 arithmetic.  The reference's own FP64 vertex-face value
+//    the inputs and of the FP32 arithmetic, at most 42 u32 L (8 measured,
+//    tests/test_certificate_band.py); L in FP32, within 3 u32 L, moves it by 2e-5 u32 L.
+//    The reference's own FP64 vertex-face value
 //    comes from a quadratic form, which may underestimate the squared distance by up to
 //    32 u64 M (M bounds the form's terms); that is subtracted too.  Result: a certified
 //    lower bound LB_f <= (reference FP64 value of feature f).
