@@ -33,13 +33,15 @@ __device__ __forceinline__ float gelu(float x) {
 __device__ __forceinline__ float gelu_grad(float x) {
   const float x2 = x * x;
   const float th = tanh_hw(x * fmaf(kGeluC * kGeluK, x2, kGeluK));
-  return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * kGeluK * fmaf(3.f * kGeluC, x2, 1.f);
+  const float sech2 = fmaf(-th, th, 1.f);
+  const float q = 0.5f * x * sech2 * kGeluK * fmaf(3.f * kGeluC, x2, 1.f);
+  return fmaf(0.5f, 1.f + th, q);
 }
 
 // gelu and gelu_grad of two values with the packed FP32 operations of sm_100 (one issue slot
-// for both; each lane rounds as the scalar operation does: gelu2 is gelu bit for bit, and gelu_grad2 spells
-// out the multiply-adds that the compiler forms in gelu_grad).
-// The tcgen05 kernels' epilogues are bound by issue slots and the tanh unit.
+// for both), the same operations in the same order: every multiply-add is written out in both
+// forms, so each lane rounds as the scalar form does.  The tcgen05 kernels' epilogues are
+// bound by issue slots and the tanh unit.
 __device__ __forceinline__ float2 splat2(float x) { return make_float2(x, x); }
 __device__ __forceinline__ float2 gelu2(float2 x) {
   const float2 u = __fmul2_rn(x, __ffma2_rn(splat2(kGeluC * kGeluK), __fmul2_rn(x, x), splat2(kGeluK)));
