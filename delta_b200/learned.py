@@ -20,7 +20,7 @@ import math
 
 import numpy as np
 
-from ._lib import check, lib
+from ._lib import ERR_UNSUPPORTED, check, lib
 from .narrowphase import BF, F64, Context, pairs_device
 
 IN, HIDDEN, OUT, FEATURES = 32, 128, 4, 18
@@ -193,16 +193,23 @@ class WarmStartMLP:
 
     def train_step(self, X, T, valid, n_valid: int, lr=1e-3):
         """forward, backward and adam.  On the tcgen05 engine one fused call
-        (delta_mlp_train_step), which leaves the forward workspaces (Z, H, Y) alone."""
+        (delta_mlp_train_step), which leaves the forward workspaces (Z, H, Y) alone; not for
+        a model whose forward, backward or adam is its own, nor for rows that are not 16-byte
+        aligned."""
         M = X.shape[0]
-        if M > 0 and getattr(self.ctx, "mlp_engine", "tcgen05") == "tcgen05" and not (X.data_ptr() | T.data_ptr()) & 15:
-            self.steps += 1
-            check(lib().delta_mlp_train_step(self.ctx.handle, M, X.data_ptr(), T.data_ptr(), valid.data_ptr(),
-                                             1.0 / max(n_valid, 1), self.params.data_ptr(),
-                                             self.params_bf16.data_ptr(), self.grads.data_ptr(), self.m.data_ptr(),
-                                             self.v.data_ptr(), lr, 0.9, 0.999, 1e-8, self.steps,
-                                             self.loss.data_ptr()))
-            return
+        own = any(getattr(getattr(self, f), "__func__", None) is not getattr(WarmStartMLP, f)
+                  for f in ("forward", "backward", "adam"))
+        if (M > 0 and not own and getattr(self.ctx, "mlp_engine", "tcgen05") == "tcgen05"
+                and not (X.data_ptr() | T.data_ptr()) & 15):
+            status = lib().delta_mlp_train_step(self.ctx.handle, M, X.data_ptr(), T.data_ptr(), valid.data_ptr(),
+                                                1.0 / max(n_valid, 1), self.params.data_ptr(),
+                                                self.params_bf16.data_ptr(), self.grads.data_ptr(), self.m.data_ptr(),
+                                                self.v.data_ptr(), lr, 0.9, 0.999, 1e-8, self.steps + 1,
+                                                self.loss.data_ptr())
+            if status != ERR_UNSUPPORTED:  # (the context's engine is another: set by delta_mlp_set_engine)
+                check(status)
+                self.steps += 1
+                return
         self.forward(X)
         self.backward(X, T, valid, n_valid)
         self.adam(lr)
