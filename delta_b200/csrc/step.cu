@@ -2274,9 +2274,10 @@ struct delta_sim {
     GraphState *state = nullptr;  // what d_nc .. d_pend point into
     int64_t *d_pend = nullptr;  // the step in flight's pairs, triangle pairs, solved pairs
     int64_t log_len = 0;
-    // the skin list (its buffer sk), its rebuilds' kernels, and the stream its conditional
-    // body is captured from
-    void *sk = nullptr;
+    void *mem = nullptr;  // the buffers above, and room for the skin list
+    // the skin list and cub's storage for it where they are longer than that room (sk, sk_temp),
+    // the kernels of its rebuilds, and the stream its conditional body is captured from
+    void *sk = nullptr, *sk_temp = nullptr;
     delta::SkinList skin{};
     int rebuild_kernels = 0;
     int skin_ctas = 8;  // k_skin_step's cluster
@@ -2405,16 +2406,17 @@ static void graph_drop_recorded(delta_sim::Graph &g) {
 
 static void graph_release(delta_sim::Graph &g) {
   graph_drop_recorded(g);
-  for (void *p : {(void *)g.pa, g.bp, g.fs, g.ds, g.temp, g.c_mem, g.dev, g.sk})
+  for (void *p : {g.mem, g.sk, g.sk_temp})
     if (p) cudaFree(p);
   g.pa = g.pb = nullptr;
-  g.bp = g.fs = g.ds = g.temp = g.c_mem = g.dev = g.sk = nullptr;
+  g.bp = g.fs = g.ds = g.temp = g.c_mem = g.dev = g.mem = g.sk = g.sk_temp = nullptr;
   g.skin = delta::SkinList{};
   g.rebuilds_seen = 0;
 }
 
 // (Re)allocates the fixed buffers for the given capacities (no capture in progress).
-static delta_status graph_alloc(delta_sim *s, int64_t pair_cap, int64_t contact_cap, int64_t log_len) {
+static constexpr int32_t kSkinRoomBodies = 1 << 15;
+static delta_status graph_alloc_all(delta_sim *s, int64_t pair_cap, int64_t contact_cap, int64_t log_len) {
   delta_sim::Graph &g = s->g;
   graph_release(g);
   const int32_t n = s->scene.n_bodies;
@@ -2425,15 +2427,37 @@ static delta_status graph_alloc(delta_sim *s, int64_t pair_cap, int64_t contact_
   size_t t = detect_fixed_temp_bytes(pair_cap, contact_cap);
   t = std::max(t, forces_fixed_temp_bytes(contact_cap, n));
   t = std::max(t, broadphase_fixed_temp_bytes(n, pair_cap));
+  // One allocation for all: of the first step of a new simulation of 16,000 bodies, seven and
+  // one for the skin list were 350 us of 1,020.  The skin list's length is known only after a
+  // search that runs in these buffers, so smaller scenes get room for five pairs a body at once
+  // (a dense packing has about three within reach).
+  const int64_t skin_room = s->plan.skin > 0.0 && n <= kSkinRoomBodies ? 1024 + 5 * (int64_t)n : 0;
+  if (skin_room > 0) t = std::max(t, skin_temp_bytes(s->scene, s->plan, skin_room));
   g.temp_bytes = t + 256;
-  const size_t cbytes = (14 * sizeof(double) + 5 * sizeof(int32_t) + 1) * (size_t)contact_cap + 256;
-  if ((e = cudaMalloc(&g.pa, sizeof(int32_t) * 2 * (size_t)pair_cap)) != cudaSuccess ||
-      (e = cudaMalloc(&g.bp, broadphase_fixed_state_bytes(n, pair_cap))) != cudaSuccess ||
-      (e = cudaMalloc(&g.fs, forces_fixed_state_bytes(contact_cap, n))) != cudaSuccess ||
-      (e = cudaMalloc(&g.ds, detect_fixed_state_bytes(pair_cap, contact_cap))) != cudaSuccess ||
-      (e = cudaMalloc(&g.temp, g.temp_bytes)) != cudaSuccess || (e = cudaMalloc(&g.c_mem, cbytes)) != cudaSuccess ||
-      (e = cudaMalloc(&g.dev, 256 + sizeof(int64_t) * (size_t)log_len)) != cudaSuccess)
-    return cuda_error(e, "graph buffers");
+  const size_t sizes[] = {sizeof(int32_t) * 2 * (size_t)pair_cap,
+                          broadphase_fixed_state_bytes(n, pair_cap),
+                          forces_fixed_state_bytes(contact_cap, n),
+                          detect_fixed_state_bytes(pair_cap, contact_cap),
+                          g.temp_bytes,
+                          (14 * sizeof(double) + 5 * sizeof(int32_t) + 1) * (size_t)contact_cap + 256,
+                          256 + sizeof(int64_t) * (size_t)log_len,
+                          skin_room > 0 ? skin_bytes(n, skin_room) + skin_build_bytes(n, skin_room) : 0};
+  void *part[8];
+  size_t total = 0;
+  for (size_t b : sizes) total += (b + 511) & ~(size_t)511;
+  if ((e = cudaMalloc(&g.mem, total)) != cudaSuccess) return cuda_error(e, "graph buffers");
+  char *at = (char *)g.mem;
+  for (int k = 0; k < 8; ++k) {
+    part[k] = at;
+    at += (sizes[k] + 511) & ~(size_t)511;
+  }
+  g.pa = (int32_t *)part[0];
+  g.bp = part[1];
+  g.fs = part[2];
+  g.ds = part[3];
+  g.temp = part[4];
+  g.c_mem = part[5];
+  g.dev = part[6];
   g.pb = g.pa + pair_cap;
   double *d = (double *)g.c_mem;
   const int64_t cap = contact_cap;
@@ -2463,15 +2487,18 @@ static delta_status graph_alloc(delta_sim *s, int64_t pair_cap, int64_t contact_
     const int64_t cap = std::max<int64_t>(1024, found + found / 2 + 1024);
     const size_t tb = skin_temp_bytes(s->scene, s->plan, cap) + 256;
     if (tb > g.temp_bytes) {
-      cudaFree(g.temp);
-      g.temp = nullptr;
-      if ((e = cudaMalloc(&g.temp, tb)) != cudaSuccess) return cuda_error(e, "skin temp");
+      if ((e = cudaMalloc(&g.sk_temp, tb)) != cudaSuccess) return cuda_error(e, "skin temp");
+      g.temp = g.sk_temp;
       g.temp_bytes = tb;
     }
     const bool cluster = skin_cluster(s->scene, s->plan, cap);
-    if ((e = cudaMalloc(&g.sk, skin_bytes(n, cap) + (cluster ? skin_build_bytes(n, cap) : 0))) != cudaSuccess)
-      return cuda_error(e, "skin list");
-    g.skin = carve_skin(g.sk, n, cap);
+    void *list = part[7];
+    if (cap > skin_room) {
+      if ((e = cudaMalloc(&g.sk, skin_bytes(n, cap) + (cluster ? skin_build_bytes(n, cap) : 0))) != cudaSuccess)
+        return cuda_error(e, "skin list");
+      list = g.sk;
+    }
+    g.skin = carve_skin(list, n, cap);
     if (cluster) {
       const SkinBuild bd = carve_skin_build(g.skin.anchor + 3 * (size_t)n, n, cap);
       if ((e = cudaMemset(bd.bcount, 0, 4 * ((size_t)bd.nb + n + 2))) != cudaSuccess ||
@@ -2482,12 +2509,19 @@ static delta_status graph_alloc(delta_sim *s, int64_t pair_cap, int64_t contact_
     g.skin.need = &g.state->need;
     g.skin.rebuilds = &g.state->rebuilds;
     // (keys: all empty until the first build, because k_skin_step tests them before it)
-    if ((e = cudaMemset(g.sk, 0, 256)) != cudaSuccess || (e = cudaMemset(g.skin.need, 0xff, sizeof(int))) != cudaSuccess ||
+    if ((e = cudaMemset(list, 0, 256)) != cudaSuccess || (e = cudaMemset(g.skin.need, 0xff, sizeof(int))) != cudaSuccess ||
         (e = cudaMemset(g.skin.keys, 0xff, sizeof(uint64_t) * (size_t)cap)) != cudaSuccess)
       return cuda_error(e, "skin init");
   }
   if ((e = cudaStreamSynchronize(s->ctx->stream)) != cudaSuccess) return cuda_error(e, "graph init");
   return DELTA_OK;
+}
+
+// The same, leaving nothing allocated when it fails (the next call allocates again).
+static delta_status graph_alloc(delta_sim *s, int64_t pair_cap, int64_t contact_cap, int64_t log_len) {
+  const delta_status st = graph_alloc_all(s, pair_cap, contact_cap, log_len);
+  if (st != DELTA_OK) graph_release(s->g);
+  return st;
 }
 
 // The step's broadphase from the skin list by one cluster, under capture on g.stream.
