@@ -2285,9 +2285,10 @@ struct delta_sim {
     cudaStream_t stream2 = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev = nullptr;
-    // the recorded step, and kGraphSteps of it in one graph (recorded when a call has as many)
+    // the recorded step, and kGraphSteps of it in one graph
     cudaGraph_t graph[2] = {nullptr, nullptr};
     cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    int64_t singles = 0;  // steps replayed one by one since the step was recorded
     delta_step_params params{};
     int kernels = 0;
     int64_t launch_epoch = 0;  // the context's launch shapes the graph was recorded with
@@ -2298,6 +2299,12 @@ struct delta_sim {
 // us (a replayed lattice step is 46); inside a graph a step's first kernel starts as a
 // dependent launch like the others.
 static constexpr int kGraphSteps = 8;
+// That graph is recorded once the steps of a call that are left and the steps replayed one by
+// one since the step was recorded are this many: recording it takes as long as it saves in
+// about 64 steps (0.25 ms; the first call of a new simulation, 9 steps of the lattice, 1.23 ms
+// with it and 0.98 without), with the conditional node in about 160 (70,000 bodies, 3.1 and
+// 2.0 ms).
+static constexpr int64_t kGraphLongAfter = 64, kGraphLongAfterNode = 160;
 
 namespace delta {
 
@@ -2402,6 +2409,7 @@ static void graph_drop_recorded(delta_sim::Graph &g) {
     g.exec[k] = nullptr;
     g.graph[k] = nullptr;
   }
+  g.singles = 0;
 }
 
 static void graph_release(delta_sim::Graph &g) {
@@ -3035,11 +3043,15 @@ delta_status delta_sim_step_graph(delta_sim *s, const delta_step_params *params,
   if ((e = cudaMemcpyAsync(g.state, host, offsetof(GraphState, rebuilds), cudaMemcpyHostToDevice, g.stream)) !=
       cudaSuccess)
     return cuda_error(e, "graph setup");
+  const int64_t long_after = g.skin.cap > 0 && !skin_cluster(s->scene, s->plan, g.skin.cap) ? kGraphLongAfterNode
+                                                                                           : kGraphLongAfter;
   int32_t base = done;  // steps completed before the current batch of launches
   while (done < nsteps) {
     const int32_t batch = nsteps - done;
     for (int32_t k = 0; k < batch;) {
-      const int which = batch - k >= kGraphSteps ? 1 : 0;
+      const bool many = g.exec[1] || batch - k + g.singles >= long_after;
+      const int which = many && batch - k >= kGraphSteps ? 1 : 0;
+      if (!which) ++g.singles;
       if (!g.exec[which] && (ds = graph_capture(s, *params, which)) != DELTA_OK) return ds;
       if ((e = cudaGraphLaunch(g.exec[which], g.stream)) != cudaSuccess) return cuda_error(e, "graph launch");
       k += which ? kGraphSteps : 1;

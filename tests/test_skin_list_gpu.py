@@ -179,20 +179,20 @@ def test_the_route_changes_with_the_bodies_and_the_obstacles(ctx):
 @pytest.mark.parametrize("kind", ["sparse", "long", "overflow"])
 def test_the_conditional_node_equals_stepping(ctx, kind):
     """The skin list's other route, over rebuilds caused by motion inside graphs of eight steps
-    and of one, with counters: more than 16,384 bodies and a short list (sorted and compacted
+    (calls of 160 and more) and of one, with counters: more than 16,384 bodies and a short list (sorted and compacted
     by one CTA); a list above 32,768 keys (sorted and selected by the whole chip); a lattice
     squeezed until its list outgrows the capacity it got from the first, empty search."""
     from delta_b200.scenarios import particle_cloud_scene
 
     rng = np.random.default_rng(31)
-    side, spacing, steps = {"sparse": (26, 0.05, 27), "long": (21, 0.0206, 27), "overflow": (26, 0.027, 115)}[kind]
+    side, spacing, steps = {"sparse": (26, 0.05, 175), "long": (21, 0.0206, 175), "overflow": (26, 0.027, 175)}[kind]
     g = (np.arange(side) - (side - 1) / 2) * spacing
     cen = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
     n = len(cen)
     if kind == "sparse":
         cen[1:400:2] = cen[0:400:2] + [0.018, 0.0, 0.0]  # 200 pairs that touch
     scene = particle_cloud_scene(cen, np.full(n, 0.0095 if kind == "overflow" else 0.01), np.full(n, 20), [], seed=9)
-    scene = moving(scene, -300.0 * cen if kind == "overflow" else rng.uniform(-20.0, 20.0, (n, 3)))
+    scene = moving(scene, -200.0 * cen if kind == "overflow" else rng.uniform(-20.0, 20.0, (n, 3)))
     skin, contacts = same_run(ctx, scene, steps)
     assert contacts > 0
     if kind == "sparse":
@@ -201,3 +201,38 @@ def test_the_conditional_node_equals_stepping(ctx, kind):
         assert skin["rebuilds"] >= 3 and skin["capacity"] > 32768, skin
     else:
         assert skin["capacity"] > 8192, skin  # grown past the first list's
+
+
+def test_calls_on_both_sides_of_the_longer_graph_equal_stepping(ctx):
+    """Eight steps are recorded as one graph once 64 steps are left or were replayed one by one:
+    calls that fall short of it, reach it, and go on with it, contacts carried over."""
+    from delta_b200.engine import Simulation, StepParams
+    from delta_b200.scenarios import lattice_scene
+
+    scene, prm, runs = lattice_scene(seed=8), StepParams.make(dt=1e-5), []
+    for graph in (False, True):
+        sim = Simulation(ctx, scene, DRV_CERT)
+        cps = [sim.step(k, prm, graph=graph) for k in (20, 17, 19, 16, 1, 9, 80)]
+        runs.append((np.concatenate(cps), sim.state(), sim.counters()))
+        sim.close()
+    (c0, s0, n0), (c1, s1, n1) = runs
+    assert np.array_equal(c0, c1) and n0 == n1 and c0.sum() > 0
+    for k in STATE:
+        assert np.array_equal(s0[k], s1[k]), k
+
+
+def test_short_calls_do_not_record_the_longer_graph(ctx):
+    """A second call of eight steps replayed them as one graph, which it had to record first
+    (with the conditional node three times the call)."""
+    from delta_b200.engine import Simulation, StepParams
+
+    scene, prm, ratio = layer(17000), StepParams.make(dt=1e-9, gravity=(0.0, 0.0, 0.0)), []
+    for _ in range(5):
+        sim, times = Simulation(ctx, scene, DRV_CERT), []
+        for _ in range(4):
+            t = time.perf_counter()
+            sim.step(8, prm, graph=True)
+            times.append(time.perf_counter() - t)
+        sim.close()
+        ratio.append(times[1] / min(times[2:]))
+    assert np.median(ratio) < 1.7, ratio
