@@ -12,10 +12,14 @@
 namespace delta {
 
 constexpr int kBlockScanThreads = 1024, kBlockScanItems = 8;
-// Up to four tiles of 8,192 entries.  (With a run of 8 entries per thread, whose 64-byte
-// strides cost the CTA's loads and stores 8 sectors a request, one full tile took 7 us of a
-// hopper step and two were slower than cub's two kernels, 5 us for 10,001 entries.)
-constexpr int64_t kBlockScanMax = 4 * (int64_t)kBlockScanThreads * kBlockScanItems;
+// Up to two tiles of 8,192 entries.  Microseconds a scan, cub's two kernels / this one (200 in
+// a row in a graph): 257 entries 2.7 / 2.1, 8,192 4.1 / 2.8, 10,001 4.1 / 4.3, 16,384 4.1 / 4.8,
+// 24,576 4.1 / 6.7, 32,768 4.1 / 8.6.  A replayed step, whose other kernels are dependent
+// launches, loses about 1 us more with cub's: of 16,000 bodies (as many counts) it takes 28.8 /
+// 28.5, of 24,000 35.8 / 37.9, of 32,000 36.0 / 40.0.  (With a run of 8 entries per thread, whose
+// 64-byte strides cost the CTA's loads and stores 8 sectors a request, one full tile took 7 us
+// of a hopper step.)
+constexpr int64_t kBlockScanMax = 2 * (int64_t)kBlockScanThreads * kBlockScanItems;
 
 // out[i] = in[0] + ... + in[i-1] (integer sums: exact in any order).  A warp takes 256
 // consecutive entries of a tile in 8 rounds of 32, so that its loads and stores are whole

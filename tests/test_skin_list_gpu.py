@@ -236,3 +236,26 @@ def test_short_calls_do_not_record_the_longer_graph(ctx):
         sim.close()
         ratio.append(times[1] / min(times[2:]))
     assert np.median(ratio) < 1.7, ratio
+
+
+@pytest.mark.parametrize("pairs", [8191, 8192, 16383, 16384, 40000])
+def test_pair_counts_are_summed_at_any_capacity(ctx, pairs):
+    """A step's contacts per pair are summed over the pair capacity and one: in one CTA, of one
+    tile or two, up to 16,384 entries, beyond by cub."""
+    from delta_b200.engine import Simulation, StepParams
+    from delta_b200.scenarios import lattice_scene
+
+    scene, prm, runs = lattice_scene(seed=9, nx=6, ny=4, nz=6), StepParams.make(dt=1e-5), []
+    for graph in (False, True):
+        sim = Simulation(ctx, scene, DRV_CERT)
+        if graph:
+            sim.set_graph_capacity(pairs, 4096)
+        cps = sim.step(20, prm, graph=graph)
+        runs.append((cps, sim.state(), sim.contacts()))
+        sim.close()
+    (c0, s0, k0), (c1, s1, k1) = runs
+    assert np.array_equal(c0, c1) and c0.sum() > 0
+    for k in STATE:
+        assert np.array_equal(s0[k], s1[k]), k
+    for k in ("depth", "master", "slave", "tri_a", "tri_b"):
+        assert np.array_equal(k0[k], k1[k]), k
