@@ -644,9 +644,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // transposed in registers) while the tensor core runs chunk i's K/16 MMAs, issued by one
 // thread and committed to the buffer's mbarrier (bounded waits).  The TMEM accumulator
 // carries the sum over the CTA's K range.  The epilogue goes through shared memory so that
-// every warp store writes 128 contiguous bytes of one output row.  With split-K each CTA writes its partial tile to a workspace
-// and k_gemm_reduce adds the partials in split order, so the result does not depend on
-// scheduling (no atomics).
+// every warp store writes 128 contiguous bytes of one output row.  With split-K each CTA
+// writes its partial tile to a workspace and k_gemm_reduce adds the partials in split order,
+// so the result does not depend on scheduling (no atomics).
 // ---------------------------------------------------------------------------------------
 constexpr int kGtRows = 128, kGtK = 64, kGtThreads = 256;
 constexpr int kGtTile = kGtRows * kGtK;             // elements of one operand chunk (16 KB)
@@ -1219,8 +1219,8 @@ __global__ void __launch_bounds__(128, 8) k_learned_refine(int64_t n, const doub
 
 inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t > 0 ? (n + t - 1) / t : 1); }
 
-// The network on `engine` (mma.sync: on features written to scratch first); with the tcgen05 engine *err_out
-// receives the device time-out flag (zeroed here, set by the kernel).
+// The network on `engine` (mma.sync: on features written to scratch first); with the tcgen05
+// engine *err_out receives the device time-out flag (zeroed here, set by the kernel).
 delta_status mlp_infer_launch(delta_ctx *ctx, int engine, int64_t n, const double *a, const double *b, int64_t ld,
                               const float *params, const void *params_bf16, float *x0, int **err_out,
                               uint32_t spin = kTcSpin, int withhold = 0) {

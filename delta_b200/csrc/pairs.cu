@@ -17,8 +17,8 @@ namespace delta {
 
 enum { M_BF = 0, M_PENALTY = 1, M_PENALTY_ITER = 2, M_GJK = 3, M_HYBRID_PAIR = 4, M_BF_CERT = 5 };
 
-// Launch bounds of the pair kernel: FP64 GJK is held to 128 registers (2^22 pairs: 1.29 ms unbounded, 1.02 at 3 blocks, 1.00 at 4, 1.11 at 5).  The FP64
-// penalty kernels are bound by the FP64 pipe (44 divisions a pair) once enough warps are
+// Launch bounds of the pair kernel: FP64 GJK is held to 128 registers (2^22 pairs: 1.29 ms
+// unbounded, 1.02 at 3 blocks, 1.00 at 4, 1.11 at 5).  The FP64 penalty kernels are bound by the FP64 pipe (44 divisions a pair) once enough warps are
 // resident: unbounded (144-176 registers) one block of 256 fitted an SM.  2^22 pairs,
 // before / 2 / 3 / 4 / 5 blocks of 128 per SM: penalty 549 / 412 / 412 / 381 / 415 us,
 // adaptive penalty 693 / 520 / 520 / 493 / 513, hybrid 551 / 529 / 416 / 433 / 559.  The
@@ -107,7 +107,8 @@ __device__ __forceinline__ void bf64_write(const xf64 pq[6], int64_t i, int64_t 
 }
 
 // A thread per pair, 8 blocks of 128 per SM (64 registers).  Bound by the FP64 pipe and the
-// lanes' divergence: 2^22 pairs 1084 us before, 762 now (92 registers: 808; 48: 859).
+// lanes' divergence: 2^22 pairs 1083 us before, 744 now (762 when 92 registers took 808 and
+// 48 took 859).
 constexpr int kBfThreads = 128;
 __global__ void __launch_bounds__(kBfThreads, 8)
     k_pairs_bf64(int64_t n, const double *__restrict__ a, const double *__restrict__ b, int64_t ld,

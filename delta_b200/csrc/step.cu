@@ -3031,7 +3031,7 @@ delta_status delta_sim_step_graph(delta_sim *s, const delta_step_params *params,
   if ((e = cudaEventRecord(g.ev, s->ctx->stream)) != cudaSuccess ||
       (e = cudaStreamWaitEvent(g.stream, g.ev, 0)) != cudaSuccess)
     return cuda_error(e, "graph order");
-  // (plain host memory: pinning it cost a new simulation's first call 3 ms, and the copies
+  // (plain host memory: pinning it cost a new simulation's first call 5 ms, and the copies
   // are of a few hundred bytes that the host waits for anyway)
   std::vector<int64_t> back((256 + sizeof(int64_t) * (size_t)nsteps) / sizeof(int64_t));
   if ((ds = copy_contacts(s->c, g.c, s->n_contacts, nullptr, g.stream)) != DELTA_OK) return ds;

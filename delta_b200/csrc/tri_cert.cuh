@@ -170,7 +170,6 @@ struct CertWarpSmem {
   double coords[32][19];
   uint16_t qs[32 * 9], qp[32 * 6];
   double rd[kCertQueue], r0[kCertQueue], r1[kCertQueue];
-  int32_t surv[64];  // particle-pair driver: B triangles that passed the box test
 };
 
 // Running minimum of one feature family, ordered by (distance, feature index): equal to

@@ -158,11 +158,11 @@ __device__ __forceinline__ R pt_tri_sq_regions(const R *V0, const R *V1, const R
   return sq;
 }
 
-// The same in FP64 (R = xf64), bit for bit the regions' results.  The regions are folded into four cases: the interior, and the three edges, each with one
-// numerator and denominator and a clamp to either end.  So a warp whose lanes fall in
-// different regions runs one division and one evaluation of the squared distance; a
-// division in every region's branch cost the FP64 bf kernel 828 us per 2^22 pairs, this
-// form 762.  Every value is formed by the operations the reference's region forms it with:
+// The same in FP64 (R = xf64), bit for bit the regions' results.  The regions are folded into
+// four cases: the interior, and the three edges, each with one numerator and denominator and
+// a clamp to either end.  So a warp whose lanes fall in different regions runs one division
+// and one evaluation of the squared distance; with a division in every region's branch the
+// FP64 bf kernel took 828 us per 2^22 pairs, with this form 762 then.  Every value is formed by the operations the reference's region forms it with:
 //   region 0        interior           s, t times 1 / det
 //   regions 5, 4a   edge t = 0         s = -d / a   in [0, 1], 0 tested first
 //   regions 3, 4b   edge s = 0         t = -e / c   in [0, 1], 0 tested first
