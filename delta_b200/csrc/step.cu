@@ -2482,7 +2482,10 @@ static delta_status graph_alloc_all(delta_sim *s, int64_t pair_cap, int64_t cont
   g.d_bp = &g.state->body_pairs;
   g.d_pend = g.state->pend;  // 3 counters of the step in flight
   g.d_log = (int64_t *)((char *)g.dev + 256);
-  if ((e = cudaMemset(g.dev, 0, 256)) != cudaSuccess) return cuda_error(e, "graph memset");
+  // (the memsets go to the context's stream, which is waited for below: one on the default
+  // stream could run after the replays, which don't wait for that stream)
+  const cudaStream_t cs = s->ctx->stream;
+  if ((e = cudaMemsetAsync(g.dev, 0, 256, cs)) != cudaSuccess) return cuda_error(e, "graph memset");
   if ((e = block_sort_prepare()) != cudaSuccess) return cuda_error(e, "pair sort attributes");
   if ((e = forces_fixed_init(s->ctx->stream, g.fs, contact_cap, n)) != cudaSuccess) return cuda_error(e, "forces init");
   delta_status ds = detect_fixed_init(s->ctx->stream, g.ds, pair_cap, contact_cap);
@@ -2509,7 +2512,7 @@ static delta_status graph_alloc_all(delta_sim *s, int64_t pair_cap, int64_t cont
     g.skin = carve_skin(list, n, cap);
     if (cluster) {
       const SkinBuild bd = carve_skin_build(g.skin.anchor + 3 * (size_t)n, n, cap);
-      if ((e = cudaMemset(bd.bcount, 0, 4 * ((size_t)bd.nb + n + 2))) != cudaSuccess ||
+      if ((e = cudaMemsetAsync(bd.bcount, 0, 4 * ((size_t)bd.nb + n + 2), cs)) != cudaSuccess ||
           (e = s->plan.n_obst > kSkinFewBoxes ? skin_cluster_size<true>(&g.skin_ctas)
                                               : skin_cluster_size<false>(&g.skin_ctas)) != cudaSuccess)
         return cuda_error(e, "skin build state");
@@ -2517,8 +2520,9 @@ static delta_status graph_alloc_all(delta_sim *s, int64_t pair_cap, int64_t cont
     g.skin.need = &g.state->need;
     g.skin.rebuilds = &g.state->rebuilds;
     // (keys: all empty until the first build, because k_skin_step tests them before it)
-    if ((e = cudaMemset(list, 0, 256)) != cudaSuccess || (e = cudaMemset(g.skin.need, 0xff, sizeof(int))) != cudaSuccess ||
-        (e = cudaMemset(g.skin.keys, 0xff, sizeof(uint64_t) * (size_t)cap)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(list, 0, 256, cs)) != cudaSuccess ||
+        (e = cudaMemsetAsync(g.skin.need, 0xff, sizeof(int), cs)) != cudaSuccess ||
+        (e = cudaMemsetAsync(g.skin.keys, 0xff, sizeof(uint64_t) * (size_t)cap, cs)) != cudaSuccess)
       return cuda_error(e, "skin init");
   }
   if ((e = cudaStreamSynchronize(s->ctx->stream)) != cudaSuccess) return cuda_error(e, "graph init");
