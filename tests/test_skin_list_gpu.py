@@ -226,16 +226,18 @@ def test_short_calls_do_not_record_the_longer_graph(ctx):
     (with the conditional node three times the call)."""
     from delta_b200.engine import Simulation, StepParams
 
-    scene, prm, ratio = layer(17000), StepParams.make(dt=1e-9, gravity=(0.0, 0.0, 0.0)), []
-    for _ in range(5):
+    scene, prm = layer(17000), StepParams.make(dt=1e-9, gravity=(0.0, 0.0, 0.0))
+    second, later = [], []
+    for _ in range(6):
         sim, times = Simulation(ctx, scene, DRV_CERT), []
         for _ in range(4):
             t = time.perf_counter()
             sim.step(8, prm, graph=True)
             times.append(time.perf_counter() - t)
         sim.close()
-        ratio.append(times[1] / min(times[2:]))
-    assert np.median(ratio) < 1.7, ratio
+        second.append(times[1])
+        later += times[2:]
+    assert min(second) < 1.7 * min(later), (second, later)
 
 
 @pytest.mark.parametrize("pairs", [8191, 8192, 16383, 16384, 40000])
